@@ -221,16 +221,15 @@ struct Mlp {
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // params, grads, Adam moments
     uint16_t *w16 = nullptr;   // bf16 W1 | W2 | W3 with padded rows (inference)
     int adam_t = 0;
-    size_t cap = 0;            // training batch capacity of the activations below
-    float *z1 = nullptr, *a1 = nullptr, *z2 = nullptr, *a2 = nullptr, *z3 = nullptr, *a3 = nullptr;
-    float *y = nullptr, *dy = nullptr, *da = nullptr, *dz = nullptr, *loss = nullptr;
+    float *partial = nullptr;  // one gradient and loss per CTA of the training kernel
+    float *loss = nullptr;
 };
 
 cudaError_t mlp_alloc(Mlp &m);
 void mlp_free(Mlp &m);
 cudaError_t mlp_sync_bf16(Mlp &m, cudaStream_t s);
 // forward + backward of one batch (X [B][80] f32 device, targets [B]):
-// gradients in m.g (zeroed first), mean squared error in *m.loss
+// gradients in m.g, mean squared error in *m.loss
 cudaError_t mlp_grad(Mlp &m, const float *X, const float *target, int B, cudaStream_t s);
 cudaError_t mlp_adam(Mlp &m, float lr, cudaStream_t s);
 cudaError_t mlp_infer_features(const Mlp &m, const float *feats, size_t n, float *out,

@@ -4,8 +4,8 @@
 //
 //   inference  BF16 tensor cores (mma.sync, FP32 accumulation), in
 //              vx_mlp_infer.cuh;
-//   training   FP32 kernels: tiled GEMM (split-K with atomics for the weight
-//              gradients), bias + GELU forward/backward, MSE loss, Adam.
+//   training   FP32: forward, loss and backward of a batch in one launch,
+//              the partial gradients added in a fixed order, Adam.
 //
 // Features (80 columns, 70 used): origin mod 64 / 64 (3), direction (3), the
 // 64 child bits of the origin chunk's tile mask (bit x + z*4 + y*16 of
@@ -32,122 +32,354 @@ __global__ void __launch_bounds__(128) k_mlp_infer(InferArgs a) {
 }
 
 // ------------------------------------------------------------- training
-// C[M][N] = sum_k A(m,k) B(k,n); A(m,k) = A[m*sam + k*sak], B likewise.
-// 64x64 tile per CTA, 16x16 threads x 4x4 outputs; blockIdx.z splits K
-// (partial sums added with atomics when split > 1; C pre-zeroed then).
-__global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float *A, long sam,
-                                               long sak, const float *B, long sbk, long sbn,
-                                               float *C, long scm, long scn, int split) {
-    __shared__ float As[16][65], Bs[16][65];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    const int kchunk = (K + split - 1) / split;
-    const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
-    float acc[4][4] = {};
-    for (int k0 = kb; k0 < ke; k0 += 16) {
-        for (int i = threadIdx.x; i < 16 * 64; i += 256) {
-            // walk the contiguous dimension fastest for coalesced loads
-            int kk, mm;
-            if (sak == 1) { kk = i & 15; mm = i >> 4; } else { kk = i >> 6; mm = i & 63; }
-            const int k = k0 + kk;
-            As[kk][mm] = (k < ke && m0 + mm < M) ? A[(long)(m0 + mm) * sam + (long)k * sak] : 0.f;
-            int kb2, nn;
-            if (sbk == 1) { kb2 = i & 15; nn = i >> 4; } else { kb2 = i >> 6; nn = i & 63; }
-            const int k2 = k0 + kb2;
-            Bs[kb2][nn] = (k2 < ke && n0 + nn < N) ? B[(long)k2 * sbk + (long)(n0 + nn) * sbn] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                av[i] = As[kk][ty * 4 + i];
-                bv[i] = Bs[kk][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] += av[i] * bv[j];
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m < M && n < N) {
-                float *c = C + (long)m * scm + (long)n * scn;
-                if (split > 1) atomicAdd(c, acc[i][j]);
-                else *c = acc[i][j];
-            }
-        }
+__device__ __forceinline__ float gelu_tanh(float x) {
+    return tanhf(0.7978845608f * (x + 0.044715f * x * x * x));
 }
-
-__device__ __forceinline__ float gelu_f(float x) {
-    return 0.5f * x * (1.0f + tanhf(0.7978845608f * (x + 0.044715f * x * x * x)));
-}
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float th = tanhf(0.7978845608f * (x + 0.044715f * x * x * x));
+// GELU (tanh form) and its derivative from th = gelu_tanh(x)
+__device__ __forceinline__ float gelu_f(float x, float th) { return 0.5f * x * (1.0f + th); }
+__device__ __forceinline__ float gelu_grad(float x, float th) {
     return 0.5f * (1.0f + th) +
            0.5f * x * (1.0f - th * th) * 0.7978845608f * (1.0f + 3.0f * 0.044715f * x * x);
 }
 
-// Z[b][j] += bias[j]; A = GELU(Z)
-__global__ void k_bias_gelu(float *Z, float *Aout, const float *bias, long n) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float z = Z[i] + bias[i & (kH - 1)];
-    Z[i] = z;
-    Aout[i] = gelu_f(z);
+// Forward, loss and backward of one batch in one launch.
+//
+// What bounds it: 1.1 GFLOP of FP32 FMA at a batch of 16,384 (15 us at the
+// device's FMA rate); the batch itself is 5 MB.  Layer by layer the same step
+// was 20 launches that carried every activation through memory, and the
+// weight gradients' reductions over the batch ran on 64 CTAs: TRAIN_BEFORE.
+//
+// One CTA per SM holds all weights in shared memory.  Its two groups of 128
+// threads take tiles of 32 samples by themselves (named barriers), so one
+// group's FMAs cover the other's barriers.  A tile's activations stay in
+// shared memory from the forward to the backward pass, GELU's derivatives in
+// the registers of the threads that need them again, and the weight
+// gradients of all a group's tiles in registers (104 of them a thread):
+// nothing but the batch is read and nothing but one partial gradient per CTA
+// is written.  k_train_reduce adds the partials in a fixed order, so the
+// gradient is the same from run to run.
+//
+// Thread (ty, tx) of a group, ty = 0..7, tx = 0..15:
+//   activations     samples 4 ty + i, columns 4 tx + j
+//   W2, W3 gradients  rows 8 ty + r, columns 4 tx + j
+//   W1 gradient       rows 8 ty + r, columns tx + 16 j
+// Weight rows are float4 columns, column c of row o kept at c ^ ((o >> 2) & 7):
+// both the forward pass (16 rows at one column) and the backward pass (16
+// columns of one row) then read without bank conflicts.
+constexpr int kTs = 32;                       // samples per tile
+constexpr int kXs = kIn + 4, kAs = kH + 4;    // row strides (floats) of X and activations
+constexpr int kWs1 = 96, kWs = kH;            // row strides of the weights
+constexpr int kGroupFloats = kTs * kXs + 4 * kTs * kAs;
+constexpr int kWeightFloats = kH * kWs1 + 2 * kH * kWs + 4 * kH + 4;
+constexpr int kTrainSmem = (kWeightFloats + 2 * kGroupFloats) * (int)sizeof(float);
+static_assert(2 * kGroupFloats >= kMlpFloats + 16 * 4 * kH, "the epilogue's merge fits");
+
+__device__ __forceinline__ void group_sync(int group) {
+    asm volatile("bar.sync %0, 128;" ::"r"(group + 1) : "memory");
+}
+__device__ __forceinline__ float at4(const float4 &v, int k) {
+    return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w));
 }
 
-// dZ = dA * GELU'(Z)
-__global__ void k_gelu_back(const float *dA, const float *Z, float *dZ, long n) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dZ[i] = dA[i] * gelu_grad(Z[i]);
-}
-
-// y = A3 . wo + bo; dY = 2 (y - target) / B; loss += (y - target)^2 / B
-__global__ void k_out_loss(const float *A3, const float *p, const float *target, int B, float *y,
-                           float *dY, float *loss) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.f;
-    if (b < B) {
-        float s = p[kBo];
-        for (int j = 0; j < kH; ++j) s += A3[(long)b * kH + j] * p[kWo + j];
-        y[b] = s;
-        const float e = s - target[b];
-        dY[b] = 2.0f * e / (float)B;
-        l = e * e / (float)B;
+// z[i][j] += sum_k A[4 ty + i][k] W[4 tx + j][k], k ascending
+template <int K, int AS, int WS>
+__device__ __forceinline__ void tile_forward(const float *A, const float *W, int ty, int tx,
+                                             float z[4][4]) {
+#pragma unroll 2
+    for (int c = 0; c < K / 4; ++c) {
+        float4 a[4], w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            a[i] = *reinterpret_cast<const float4 *>(A + (4 * ty + i) * AS + 4 * c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            w[j] = *reinterpret_cast<const float4 *>(W + (4 * tx + j) * WS + 4 * (c ^ (tx & 7)));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) z[i][j] += at4(a[i], k) * at4(w[j], k);
     }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xFFFFFFFFu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, l);
 }
-
-// dA3[b][j] = dY[b] wo[j]; g_wo[j] += sum_b dY[b] A3[b][j]; g_bo += sum_b dY[b]
-// (blockDim 256 = 4 samples x 64 columns)
-__global__ void k_out_back(const float *A3, const float *dY, const float *p, int B, float *dA3,
-                           float *grad) {
-    const int j = threadIdx.x & 63;
-    float gw = 0.f, gb = 0.f;
-    for (int b = blockIdx.x * 4 + (threadIdx.x >> 6); b < B; b += gridDim.x * 4) {
-        dA3[(long)b * kH + j] = dY[b] * p[kWo + j];
-        gw += dY[b] * A3[(long)b * kH + j];
-        if (j == 0) gb += dY[b];
+// d[i][j] = sum_o dZ[4 ty + i][o] W[o][4 tx + j], o ascending
+__device__ __forceinline__ void tile_backward(const float *dZ, const float *W, int ty, int tx,
+                                              float d[4][4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[i][j] = 0.f;
+#pragma unroll 2
+    for (int c = 0; c < kH / 4; ++c) {
+        float4 a[4], w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            a[i] = *reinterpret_cast<const float4 *>(dZ + (4 * ty + i) * kAs + 4 * c);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            w[k] = *reinterpret_cast<const float4 *>(W + (4 * c + k) * kWs + 4 * (tx ^ (c & 7)));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) d[i][j] += at4(a[i], k) * at4(w[k], j);
     }
-    atomicAdd(grad + kWo + j, gw);
-    if (j == 0) atomicAdd(grad + kBo, gb);
+}
+// g[r][j] += sum_b dZ[b][8 ty + r] A[b][4 tx + j], b ascending
+__device__ __forceinline__ void tile_weight_grad(const float *dZ, const float *A, int ty, int tx,
+                                                 float g[8][4]) {
+#pragma unroll 2
+    for (int b = 0; b < kTs; ++b) {
+        const float4 z0 = *reinterpret_cast<const float4 *>(dZ + b * kAs + 8 * ty);
+        const float4 z1 = *reinterpret_cast<const float4 *>(dZ + b * kAs + 8 * ty + 4);
+        const float4 a = *reinterpret_cast<const float4 *>(A + b * kAs + 4 * tx);
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) g[r][j] += at4(r < 4 ? z0 : z1, r & 3) * at4(a, j);
+    }
 }
 
-// column sums of dZ [B][64] into grad[off + j]
-__global__ void k_bias_grad(const float *dZ, int B, float *grad, int off) {
-    const int j = threadIdx.x & 63;
-    float s = 0.f;
-    for (int b = blockIdx.x * 4 + (threadIdx.x >> 6); b < B; b += gridDim.x * 4)
-        s += dZ[(long)b * kH + j];
-    atomicAdd(grad + off + j, s);
+// partial: gridDim.x x (kMlpFloats + 1) floats, each CTA's gradient and loss
+__global__ void __launch_bounds__(256, 1) k_train_grad(const float *__restrict__ p,
+                                                       const float *__restrict__ X,
+                                                       const float *__restrict__ target, int B,
+                                                       float *__restrict__ partial) {
+    extern __shared__ __align__(16) float sm[];
+    float *sW1 = sm, *sW2 = sW1 + kH * kWs1, *sW3 = sW2 + kH * kWs, *sV = sW3 + kH * kWs;
+    const int tid = threadIdx.x, group = tid >> 7, t = tid & 127, ty = t >> 4, tx = t & 15;
+    float *gs = sm + kWeightFloats + group * kGroupFloats;
+    float *sX = gs, *sA1 = sX + kTs * kXs, *sA2 = sA1 + kTs * kAs, *sP = sA2 + kTs * kAs,
+          *sQ = sP + kTs * kAs;
+    for (int i = tid; i < kH * kIn / 4; i += 256) {
+        const int o = i / (kIn / 4), c = i % (kIn / 4);
+        *reinterpret_cast<float4 *>(sW1 + o * kWs1 + 4 * (c ^ ((o >> 2) & 7))) =
+            *reinterpret_cast<const float4 *>(p + kW1 + 4 * i);
+    }
+    for (int i = tid; i < kH * kH / 4; i += 256) {
+        const int o = i >> 4, c = i & 15, at = o * kWs + 4 * (c ^ ((o >> 2) & 7));
+        *reinterpret_cast<float4 *>(sW2 + at) = *reinterpret_cast<const float4 *>(p + kW2 + 4 * i);
+        *reinterpret_cast<float4 *>(sW3 + at) = *reinterpret_cast<const float4 *>(p + kW3 + 4 * i);
+    }
+    // b1, b2, b3, wo, bo
+    if (tid < kH) {
+        sV[tid] = p[kB1 + tid];
+        sV[kH + tid] = p[kB2 + tid];
+        sV[2 * kH + tid] = p[kB3 + tid];
+        sV[3 * kH + tid] = p[kWo + tid];
+        if (tid == 0) sV[4 * kH] = p[kBo];
+    }
+    __syncthreads();
+
+    float g1[8][5] = {}, g2[8][4] = {}, g3[8][4] = {};
+    float gb1[4] = {}, gb2[4] = {}, gb3[4] = {}, gwo[4] = {}, gbo = 0.f, loss = 0.f;
+    const bool wide = (reinterpret_cast<uintptr_t>(X) & 15u) == 0u;
+    const int tiles = (B + kTs - 1) / kTs;
+    // consecutive tiles go to different SMs, then to the second groups
+    for (int tile = blockIdx.x + group * gridDim.x; tile < tiles; tile += 2 * gridDim.x) {
+        const int b0 = tile * kTs, rows = min(kTs, B - b0);
+        // samples beyond the batch are zero rows and get a zero dY
+        if (wide) {
+#pragma unroll
+            for (int k = 0; k < kTs * kIn / 4 / 128; ++k) {
+                const int i = t + 128 * k, r = i / (kIn / 4), c = i % (kIn / 4);
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < rows) v = __ldg(reinterpret_cast<const float4 *>(X + (size_t)(b0 + r) * kIn) + c);
+                *reinterpret_cast<float4 *>(sX + r * kXs + 4 * c) = v;
+            }
+        } else {
+            for (int i = t; i < kTs * kIn; i += 128) {
+                const int r = i / kIn, c = i % kIn;
+                sX[r * kXs + c] = r < rows ? __ldg(X + (size_t)(b0 + r) * kIn + c) : 0.f;
+            }
+        }
+        group_sync(group);
+        float z[4][4], d1[4][4], d2[4][4];
+        // layers 1 and 2: activations to shared memory, derivatives kept
+#pragma unroll
+        for (int layer = 0; layer < 2; ++layer) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) z[i][j] = 0.f;
+            if (layer == 0) tile_forward<kIn, kXs, kWs1>(sX, sW1, ty, tx, z);
+            else tile_forward<kH, kAs, kWs>(sA1, sW2, ty, tx, z);
+            float *out = layer == 0 ? sA1 : sA2;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float x = z[i][j] + sV[layer * kH + 4 * tx + j], th = gelu_tanh(x);
+                    v[j] = gelu_f(x, th);
+                    (layer == 0 ? d1 : d2)[i][j] = gelu_grad(x, th);
+                }
+                *reinterpret_cast<float4 *>(out + (4 * ty + i) * kAs + 4 * tx) =
+                    make_float4(v[0], v[1], v[2], v[3]);
+            }
+            group_sync(group);
+        }
+        // layer 3, the output and the loss: y = A3 . wo + bo, dY = 2 (y - target) / B
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) z[i][j] = 0.f;
+        tile_forward<kH, kAs, kWs>(sA2, sW3, ty, tx, z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = 4 * ty + i;
+            float a3[4], d3[4], y = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float x = z[i][j] + sV[2 * kH + 4 * tx + j], th = gelu_tanh(x);
+                a3[j] = gelu_f(x, th);
+                d3[j] = gelu_grad(x, th);
+                y += a3[j] * sV[3 * kH + 4 * tx + j];
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) y += __shfl_xor_sync(0xFFFFFFFFu, y, o);
+            float dy = 0.f;
+            if (r < rows) {
+                const float e = (y + sV[4 * kH]) - __ldg(target + b0 + r);
+                dy = 2.0f * e / (float)B;
+                if (tx == 0) {
+                    loss += e * e / (float)B;
+                    gbo += dy;
+                }
+            }
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                gwo[j] += dy * a3[j];
+                v[j] = dy * sV[3 * kH + 4 * tx + j] * d3[j];
+                gb3[j] += v[j];
+            }
+            *reinterpret_cast<float4 *>(sP + r * kAs + 4 * tx) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+        group_sync(group);
+        // backward: dZ3 in sP, dZ2 in sQ, dZ1 in sP
+        tile_weight_grad(sP, sA2, ty, tx, g3);
+        tile_backward(sP, sW3, ty, tx, z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                z[i][j] *= d2[i][j];
+                gb2[j] += z[i][j];
+            }
+            *reinterpret_cast<float4 *>(sQ + (4 * ty + i) * kAs + 4 * tx) =
+                make_float4(z[i][0], z[i][1], z[i][2], z[i][3]);
+        }
+        group_sync(group);
+        tile_weight_grad(sQ, sA1, ty, tx, g2);
+        tile_backward(sQ, sW2, ty, tx, z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                z[i][j] *= d1[i][j];
+                gb1[j] += z[i][j];
+            }
+            *reinterpret_cast<float4 *>(sP + (4 * ty + i) * kAs + 4 * tx) =
+                make_float4(z[i][0], z[i][1], z[i][2], z[i][3]);
+        }
+        group_sync(group);
+#pragma unroll 2
+        for (int b = 0; b < kTs; ++b) {
+            const float4 z0 = *reinterpret_cast<const float4 *>(sP + b * kAs + 8 * ty);
+            const float4 z1 = *reinterpret_cast<const float4 *>(sP + b * kAs + 8 * ty + 4);
+#pragma unroll
+            for (int j = 0; j < 5; ++j) {
+                const float x = sX[b * kXs + tx + 16 * j];
+#pragma unroll
+                for (int r = 0; r < 8; ++r) g1[r][j] += at4(r < 4 ? z0 : z1, r & 3) * x;
+            }
+        }
+        group_sync(group);
+    }
+
+    // the CTA's partial: group 1's sums through shared memory, group 0 adds
+    // its own; the column sums (biases, wo) of the 16 (group, ty) rows after
+    __syncthreads();
+    float *mg = sm + kWeightFloats, *cols = mg + kMlpFloats;
+    float *out = partial + (size_t)blockIdx.x * (kMlpFloats + 1);
+#pragma unroll
+    for (int phase = 0; phase < 2; ++phase) {
+        if (group == 1 - phase) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+#pragma unroll
+                for (int j = 0; j < 5; ++j) {
+                    const int i = kW1 + (8 * ty + r) * kIn + tx + 16 * j;
+                    if (phase == 0) mg[i] = g1[r][j];
+                    else out[i] = g1[r][j] + mg[i];
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int i = (8 * ty + r) * kH + 4 * tx + j;
+                    if (phase == 0) {
+                        mg[kW2 + i] = g2[r][j];
+                        mg[kW3 + i] = g3[r][j];
+                    } else {
+                        out[kW2 + i] = g2[r][j] + mg[kW2 + i];
+                        out[kW3 + i] = g3[r][j] + mg[kW3 + i];
+                    }
+                }
+            }
+        }
+        if (phase == 0) {
+            float *c = cols + (group * 8 + ty) * 4 * kH + 4 * tx;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                c[j] = gb1[j];
+                c[kH + j] = gb2[j];
+                c[2 * kH + j] = gb3[j];
+                c[3 * kH + j] = gwo[j];
+            }
+            if (tx == 0) {
+                sV[group * 8 + ty] = gbo;
+                sV[16 + group * 8 + ty] = loss;
+            }
+        }
+        __syncthreads();
+    }
+    {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s += cols[k * 4 * kH + tid];
+        const int off[4] = {kB1, kB2, kB3, kWo};
+        out[off[tid >> 6] + (tid & 63)] = s;
+        if (tid < 2) {
+            float v = 0.f;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v += sV[16 * tid + k];
+            out[tid == 0 ? kBo : kMlpFloats] = v;
+        }
+    }
+}
+
+// grad[i] (and the loss, entry kMlpFloats) = sum of the partials in CTA order:
+// 32 entries per CTA, eight threads each take every eighth partial.
+__global__ void __launch_bounds__(256) k_train_reduce(const float *__restrict__ partial, int parts,
+                                                      float *__restrict__ grad,
+                                                      float *__restrict__ loss) {
+    __shared__ float s[8][33];
+    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    float v = 0.f;
+    if (i <= kMlpFloats) {
+#pragma unroll 8
+        for (int c = row; c < parts; c += 8) v += __ldg(partial + (size_t)c * (kMlpFloats + 1) + i);
+    }
+    s[row][lane] = v;
+    __syncthreads();
+    if (row == 0 && i <= kMlpFloats) {
+#pragma unroll
+        for (int k = 1; k < 8; ++k) v += s[k][lane];
+        if (i < kMlpFloats) grad[i] = v;
+        else *loss = v;
+    }
 }
 
 __global__ void k_adam(float *p, const float *g, float *m, float *v, int n, float lr, float b1,
@@ -248,27 +480,10 @@ cudaError_t mlp_alloc(Mlp &m) {
 }
 
 void mlp_free(Mlp &m) {
-    for (float *q : {m.p, m.g, m.m, m.v, m.z1, m.a1, m.z2, m.a2, m.z3, m.a3, m.y, m.dy, m.da,
-                     m.dz, m.loss})
+    for (float *q : {m.p, m.g, m.m, m.v, m.partial, m.loss})
         if (q) cudaFree(q);
     if (m.w16) cudaFree(m.w16);
     m = Mlp();
-}
-
-static cudaError_t mlp_reserve(Mlp &m, size_t B) {
-    if (m.cap >= B) return cudaSuccess;
-    for (float **q : {&m.z1, &m.a1, &m.z2, &m.a2, &m.z3, &m.a3, &m.da, &m.dz, &m.y, &m.dy}) {
-        if (*q) cudaFree(*q);
-        *q = nullptr;
-    }
-    m.cap = 0;
-    cudaError_t e = cudaSuccess;
-    for (float **q : {&m.z1, &m.a1, &m.z2, &m.a2, &m.z3, &m.a3, &m.da, &m.dz})
-        if (e == cudaSuccess) e = cudaMalloc(q, B * kH * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m.y, B * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m.dy, B * sizeof(float));
-    if (e == cudaSuccess) m.cap = B;
-    return e;
 }
 
 cudaError_t mlp_sync_bf16(Mlp &m, cudaStream_t s) {
@@ -278,40 +493,18 @@ cudaError_t mlp_sync_bf16(Mlp &m, cudaStream_t s) {
 
 cudaError_t mlp_grad(Mlp &m, const float *X, const float *target, int B, cudaStream_t s) {
     if (B <= 0) return cudaErrorInvalidValue;
-    cudaError_t e = mlp_reserve(m, (size_t)B);
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess && !m.partial)
+        e = cudaMalloc(&m.partial, (size_t)sms * (kMlpFloats + 1) * sizeof(float));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_train_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kTrainSmem);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(m.g, 0, kMlpFloats * sizeof(float), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m.loss, 0, sizeof(float), s);
-    if (e != cudaSuccess) return e;
-    const long n = (long)B * kH;
-    auto gemm = [&](int M, int N, int K, const float *A, long sam, long sak, const float *Bm,
-                    long sbk, long sbn, float *C, long scm, long scn, int split) {
-        const dim3 grid((N + 63) / 64, (M + 63) / 64, split);
-        k_sgemm<<<grid, 256, 0, s>>>(M, N, K, A, sam, sak, Bm, sbk, sbn, C, scm, scn, split);
-    };
-    const unsigned bb = std::min<unsigned>(nblk((size_t)B, 4), 1184u);
-    // forward: Z = X W^T (+ b), A = GELU(Z)
-    gemm(B, kH, kIn, X, kIn, 1, m.p + kW1, 1, kIn, m.z1, kH, 1, 1);
-    k_bias_gelu<<<nblk(n, 256), 256, 0, s>>>(m.z1, m.a1, m.p + kB1, n);
-    gemm(B, kH, kH, m.a1, kH, 1, m.p + kW2, 1, kH, m.z2, kH, 1, 1);
-    k_bias_gelu<<<nblk(n, 256), 256, 0, s>>>(m.z2, m.a2, m.p + kB2, n);
-    gemm(B, kH, kH, m.a2, kH, 1, m.p + kW3, 1, kH, m.z3, kH, 1, 1);
-    k_bias_gelu<<<nblk(n, 256), 256, 0, s>>>(m.z3, m.a3, m.p + kB3, n);
-    k_out_loss<<<nblk((size_t)B, 256), 256, 0, s>>>(m.a3, m.p, target, B, m.y, m.dy, m.loss);
-    // backward (weight gradients: split-K over the batch)
-    const int split = std::max(1, std::min(148, B / 256));
-    k_out_back<<<bb, 256, 0, s>>>(m.a3, m.dy, m.p, B, m.da, m.g);
-    k_gelu_back<<<nblk(n, 256), 256, 0, s>>>(m.da, m.z3, m.dz, n);              // dZ3
-    gemm(kH, kH, B, m.dz, 1, kH, m.a2, kH, 1, m.g + kW3, kH, 1, split);         // gW3 = dZ3^T A2
-    k_bias_grad<<<bb, 256, 0, s>>>(m.dz, B, m.g, kB3);
-    gemm(B, kH, kH, m.dz, kH, 1, m.p + kW3, kH, 1, m.da, kH, 1, 1);             // dA2 = dZ3 W3
-    k_gelu_back<<<nblk(n, 256), 256, 0, s>>>(m.da, m.z2, m.dz, n);              // dZ2
-    gemm(kH, kH, B, m.dz, 1, kH, m.a1, kH, 1, m.g + kW2, kH, 1, split);
-    k_bias_grad<<<bb, 256, 0, s>>>(m.dz, B, m.g, kB2);
-    gemm(B, kH, kH, m.dz, kH, 1, m.p + kW2, kH, 1, m.da, kH, 1, 1);             // dA1 = dZ2 W2
-    k_gelu_back<<<nblk(n, 256), 256, 0, s>>>(m.da, m.z1, m.dz, n);              // dZ1
-    gemm(kH, kIn, B, m.dz, 1, kH, X, kIn, 1, m.g + kW1, kIn, 1, split);         // gW1 = dZ1^T X
-    k_bias_grad<<<bb, 256, 0, s>>>(m.dz, B, m.g, kB1);
+    const int grid = std::min(sms, (B + kTs - 1) / kTs);
+    k_train_grad<<<grid, 256, kTrainSmem, s>>>(m.p, X, target, B, m.partial);
+    k_train_reduce<<<nblk(kMlpFloats + 1, 32), 256, 0, s>>>(m.partial, grid, m.g, m.loss);
     return cudaGetLastError();
 }
 
