@@ -52,6 +52,7 @@ struct VxWorld {
         VxPickHit out;
         int32_t hit;
         uint32_t fault;               // DevWorld::fault (kFaultBeamCopyLost)
+        uint32_t masks_bad;           // answer of launch_masks_hold
     };
     PickBox *pick = nullptr;          // host address
     PickBox *pick_dev = nullptr;      // device address of the same block
@@ -104,6 +105,11 @@ struct VxWorld {
     // the masks changed (mask_gen) since they were built (df_gen)
     uint8_t *bdf = nullptr, *tdf = nullptr, *df_tmp = nullptr;
     std::atomic<uint64_t> mask_gen{1};
+    // every brick with a solid voxel is under set mask bits: so by
+    // construction wherever the library builds the masks (updates of part of
+    // them keep it), checked where the caller uploads them.  Batched picking
+    // skips by the masks then, as raycast() itself does not read them.
+    std::atomic<bool> masks_hold{true};
     uint64_t df_gen = 0;
     float *lrn_depth = nullptr;      // per-tile proven depths of learned frames without a proposal
     size_t lrn_depth_cap = 0;
@@ -511,6 +517,7 @@ int vx_world_upload(VxWorld *w, const VxBrick *bricks, const uint64_t *tile_mask
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
     forget_generated(w);
+    w->masks_hold = false;
     const vx::Dims &d = w->dw.d;
     const size_t chunk = (size_t)1 << 20;  // bricks per staging round (72 MiB)
     rc = ensure(&w->d_bricks, &w->bricks_cap, std::min<size_t>(chunk, (size_t)d.n_bricks));
@@ -528,7 +535,10 @@ int vx_world_upload(VxWorld *w, const VxBrick *bricks, const uint64_t *tile_mask
     VX_CK(cudaMemcpyAsync(w->dw.tile_uniform, tile_uniform, d.n_tiles, cudaMemcpyHostToDevice, w->stream));
     vx::world_masks_changed(w);
     VX_CK(vx::launch_tile_meta(w->dw, w->stream));
+    w->pick->masks_bad = 0u;
+    VX_CK(vx::launch_masks_hold(w->dw, &w->pick_dev->masks_bad, w->stream));
     VX_CK(cudaStreamSynchronize(w->stream));
+    w->masks_hold = *const_cast<volatile uint32_t *>(&w->pick->masks_bad) == 0u;
     return VX_OK;
 }
 
@@ -571,6 +581,7 @@ int vx_world_generate(VxWorld *w, const VxTerrainParams *t) {
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
     forget_generated(w);
+    w->masks_hold = false;
     const vx::Dims &d = w->dw.d;
     int16_t *heights = nullptr;
     VX_CK(cudaMallocAsync(&heights, (size_t)d.vx * d.vz * sizeof(int16_t), w->stream));
@@ -579,6 +590,7 @@ int vx_world_generate(VxWorld *w, const VxTerrainParams *t) {
     cudaFreeAsync(heights, w->stream);
     VX_CK(e);
     VX_CK(cudaStreamSynchronize(w->stream));
+    w->masks_hold = true;
     return VX_OK;
 }
 
@@ -741,6 +753,7 @@ int run_gen_plan(VxWorld *w, uint64_t seed, vx::GenPlan &plan, const std::vector
     vx::world_masks_changed(w);
     VX_CK(vx::launch_gen_slots(w->dw, seed, plan, w->stream));
     VX_CK(cudaStreamSynchronize(w->stream));
+    w->masks_hold = true;            // every mask was rebuilt
     return VX_OK;
 }
 
@@ -1242,7 +1255,7 @@ int vx_raycast_batch(VxWorld *w, const int32_t origin[3], const float *cams_dev,
     int rc = use_device(w);
     if (rc != VX_OK) return rc;
     VX_CK(vx::launch_raycast(w->dw, origin, cams_dev, dirs_dev, n, out_dev, hit_dev,
-                             as_stream(stream)));
+                             w->masks_hold, as_stream(stream)));
     return VX_OK;
 }
 
