@@ -110,6 +110,7 @@ struct VxWorld {
     // them keep it), checked where the caller uploads them.  Batched picking
     // skips by the masks then, as raycast() itself does not read them.
     std::atomic<bool> masks_hold{true};
+    bool tiles_built = true;         // tile words and LUT bytes are the library's, for every tile
     uint64_t df_gen = 0;
     float *lrn_depth = nullptr;      // per-tile proven depths of learned frames without a proposal
     size_t lrn_depth_cap = 0;
@@ -518,6 +519,7 @@ int vx_world_upload(VxWorld *w, const VxBrick *bricks, const uint64_t *tile_mask
     std::lock_guard<std::mutex> lk(w->mu);
     forget_generated(w);
     w->masks_hold = false;
+    w->tiles_built = false;
     const vx::Dims &d = w->dw.d;
     const size_t chunk = (size_t)1 << 20;  // bricks per staging round (72 MiB)
     rc = ensure(&w->d_bricks, &w->bricks_cap, std::min<size_t>(chunk, (size_t)d.n_bricks));
@@ -591,6 +593,7 @@ int vx_world_generate(VxWorld *w, const VxTerrainParams *t) {
     VX_CK(e);
     VX_CK(cudaStreamSynchronize(w->stream));
     w->masks_hold = true;
+    w->tiles_built = true;
     return VX_OK;
 }
 
@@ -751,9 +754,10 @@ int run_gen_plan(VxWorld *w, uint64_t seed, vx::GenPlan &plan, const std::vector
     if (rc != VX_OK) return rc;
     plan.lmx = w->d_lmx;
     vx::world_masks_changed(w);
-    VX_CK(vx::launch_gen_slots(w->dw, seed, plan, w->stream));
+    VX_CK(vx::launch_gen_slots(w->dw, seed, plan, w->tiles_built, w->stream));
     VX_CK(cudaStreamSynchronize(w->stream));
     w->masks_hold = true;            // every mask was rebuilt
+    w->tiles_built = true;
     return VX_OK;
 }
 
@@ -955,8 +959,9 @@ int vx_world_shift_origin(VxWorld *w, int32_t origin_cx, int32_t origin_cz,
     const vx::Dims &d = w->dw.d;
     const int32_t sx_n = d.bx / 8, sy_n = d.by / 8, sz_n = d.bz / 8;
     std::vector<int32_t> chunks;
-    for (int32_t sz = 0; sz < sz_n; ++sz)
-        for (int32_t sy = 0; sy < sy_n; ++sy)
+    // y slowest: the chunks below ground, which take longest, start first
+    for (int32_t sy = 0; sy < sy_n; ++sy)
+        for (int32_t sz = 0; sz < sz_n; ++sz)
             for (int32_t sx = 0; sx < sx_n; ++sx) {
                 int32_t c[3];
                 wanted_chunk(d, origin_cx, origin_cz, sx, sy, sz, c);

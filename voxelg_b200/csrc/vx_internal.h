@@ -163,10 +163,14 @@ size_t gen_prim_bytes_per_src();
 // the generator's powf / cosf / sinf (vx_gmath.h function fn) on n inputs
 cudaError_t launch_gen_math(const uint32_t *lmx, uint32_t fn, const float *in, size_t n, float *out,
                             cudaStream_t s);
-cudaError_t launch_gen_slots(const DevWorld &w, uint64_t seed, const GenPlan &p, cudaStream_t s);
+// tiles_built: every tile word and LUT byte is the one its bricks give, so
+// only the generated chunks' (which their kernel writes) change
+cudaError_t launch_gen_slots(const DevWorld &w, uint64_t seed, const GenPlan &p, bool tiles_built,
+                             cudaStream_t s);
 cudaError_t launch_generate(const DevWorld &w, const VxTerrainParams &t, int16_t *heights,
                             cudaStream_t s);
-cudaError_t launch_rebuild_pyramid(const DevWorld &w, cudaStream_t s);
+// chunk and L4 words and tile_meta, after the tiles' where `tiles`
+cudaError_t launch_rebuild_pyramid(const DevWorld &w, bool tiles, cudaStream_t s);
 // the brick and tile distance fields of w (tmp: n_bricks bytes of scratch)
 // a frame's records (and shadow records, or nullptr) [first, first + n) in
 // the 16-byte packed form (vx_pack.cu)

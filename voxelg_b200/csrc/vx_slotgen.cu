@@ -6,25 +6,34 @@
 //
 // The reference recomputes, for every storage chunk, the terrain of its
 // 32x32 columns and the trees of its 3x3 neighbourhood.  Both depend only on
-// x and z, so a batch of chunks is generated by three kernels:
-//   k_gen_columns  one thread per column of each distinct xz chunk:
+// x and z, so a batch of chunks is generated by two kernels:
+//   k_gen_xz       one thread per column of each distinct xz chunk --
 //                  sample_terrain (:1244-1316), the biome (:1342-1344) and
-//                  the surface decoration (:1394-1459) packed in one word;
-//   k_gen_trees    one thread per tree candidate of each distinct source
+//                  the surface decoration (:1394-1459) packed in one word --
+//                  and one thread per tree candidate of each distinct source
 //                  chunk (trees_for_chunk, :1537-1591), expanded into its
 //                  paint primitives (paint_tree, :1605-1710);
 //   k_gen_slot     one 256-thread CTA per storage chunk, four per SM: the
-//                  voxels of its columns (cave and ore noise per voxel) in
-//                  shared memory, then the primitives of the 3x3 source
-//                  chunks in the reference's order -- source chunk (z, x),
-//                  tree, primitive -- one primitive at a time with a
-//                  barrier between, skipping primitives whose box misses
-//                  the chunk.  Every write of one primitive carries one
-//                  material, so the order among its voxels cannot change
-//                  what try_write_tree_voxel (:1500-1525) leaves.  Last the
-//                  512 bricks, their occupancy words (occupancy == material
-//                  != 0, the invariant Brick::set keeps, :315-325) and
-//                  uniform bytes go to the slot's bricks.
+//                  voxels of its columns in shared memory (ore noise from
+//                  tables of the chunk's lattice hashes), then the
+//                  primitives of the 3x3 source chunks in the reference's
+//                  order -- source chunk (z, x), tree, primitive.  Each warp
+//                  paints a slab of four z levels by itself: it takes the
+//                  primitives that reach the slab in order, and every write
+//                  of one primitive carries one material, so the order among
+//                  its voxels cannot change what try_write_tree_voxel
+//                  (:1500-1525) leaves.  Last the 512 bricks, their occupancy
+//                  words (occupancy == material != 0, the invariant
+//                  Brick::set keeps, :315-325) and uniform bytes go to the
+//                  slot's bricks, and the chunk's eight tile words and LUT
+//                  bytes with them.
+// What bounds k_gen_slot: the ore noise of the voxels below ground (two value
+// noises each) and, before, the walk over the trees.  For a window of
+// 2048x256x2048 moved by (8, 3) chunks, 5,440 of them: 630-700 us with the
+// noise hashed column by column (526 M warp instructions), all 256 threads on
+// one primitive at a time behind a barrier and the 108 tree headers read one
+// after the other; 620 us with the lattice tables, 455 us with the slabs,
+// 392 us with the chunks below ground started first (288 M).
 // powf, cosf and sinf give the host C library's binary32 results, as the
 // reference's f32::powf / cos / sin do: vx_gmath.h's functions, corrected
 // by the exception table (Seed::lmx) on the generator's domains.
@@ -95,8 +104,13 @@ __device__ int32_t sample_terrain(float wx, float wz, float offx, float offz, co
     const float base = fbm_2d(wpx * 0.012f, wpz * 0.012f, 4) * 22.0f;
     const float mountain_mask = fmaxr(fbm_2d(wpx * 0.0028f, wpz * 0.0028f, 2) + 0.2f, 0.0f);
     const float mountain_amp = fminr(mountain_mask, 1.0f);
-    const float mountain_h =
-        pow115(lmx, fmaxr(fbm_2d(wpx * 0.009f, wpz * 0.009f, 5), 0.0f)) * mountain_amp * 110.0f;
+    // both factors are finite and not negative, so a zero one makes the
+    // product +0 whatever the other is
+    float mountain_h = 0.0f;
+    if (mountain_amp > 0.0f) {
+        const float m = fmaxr(fbm_2d(wpx * 0.009f, wpz * 0.009f, 5), 0.0f);
+        if (m > 0.0f) mountain_h = pow115(lmx, m) * mountain_amp * 110.0f;
+    }
     const float base_h = 64.0f + 8.0f + base + mountain_h - 0.0f;
     const float h = base_h < 2.0f ? 2.0f : (base_h > 255.0f ? 255.0f : base_h);
     const int32_t hi = f2i(h);
@@ -203,7 +217,7 @@ __device__ bool tree_candidate(int32_t cx, int32_t cz, uint32_t i, const Seed &g
 }
 
 enum : uint32_t { PR_LINE = 0, PR_SHELL = 1, PR_SPHERE = 2 };
-struct Prim {
+struct __align__(16) Prim {
     int32_t a[3];    // line start / shell or sphere centre
     int32_t b[3];    // line end; b[0] = radius of a shell or sphere
     uint32_t kind_mat;
@@ -241,14 +255,13 @@ struct Emit {
     }
 };
 
-// Whether a primitive can write into the chunk [lo, lo + 32): its voxels
-// lie in the box of the segment (rounding a + d t with t in [0, 1] stays
-// between the ends), in c +- (r + 1, r, r + 1) for a shell, c +- r for a
-// sphere.
-__device__ __forceinline__ bool prim_meets(const Prim &p, const int32_t lo[3]) {
+// The box of the voxels a primitive can write: its segment (rounding a + d t
+// with t in [0, 1] stays between the ends), c +- (r + 1, r, r + 1) for a
+// shell, c +- r for a sphere.
+__device__ __forceinline__ void prim_box(const Prim &p, int32_t mn[3], int32_t mx[3]) {
     const uint32_t kind = p.kind_mat >> 8;
-    int32_t mn[3], mx[3];
     if (kind == PR_LINE) {
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
             mn[k] = min(p.a[k], p.b[k]);
             mx[k] = max(p.a[k], p.b[k]);
@@ -259,9 +272,11 @@ __device__ __forceinline__ bool prim_meets(const Prim &p, const int32_t lo[3]) {
         mn[1] = p.a[1] - r;  mx[1] = p.a[1] + r;
         mn[2] = p.a[2] - rh; mx[2] = p.a[2] + rh;
     }
-    return mx[0] >= lo[0] && mn[0] < lo[0] + kCV && mx[1] >= lo[1] && mn[1] < lo[1] + kCV &&
-           mx[2] >= lo[2] && mn[2] < lo[2] + kCV;
 }
+// A tree's voxels lie within kTreeReach of its base in x and z: the longest
+// branch (5) and the shell of a branch canopy (radius 3 + 1, widened by 1);
+// pine canopies reach 4 + 1 + 1, cactus arms 2.
+constexpr int32_t kTreeReach = 10;
 
 // branch_jitter, voxel.rs:1791-1797
 __device__ __forceinline__ float branch_jitter(uint32_t hash, uint32_t b) {
@@ -331,48 +346,52 @@ __device__ void tree_prims(const Tree &t, const uint32_t *lmx, Emit &e) {
     }
 }
 
-// try_write_tree_voxel, voxel.rs:1500-1525, on the shared chunk
-__device__ __forceinline__ void tree_voxel(uint8_t *s_mat, const int32_t lo[3], int32_t x,
-                                           int32_t y, int32_t z, uint8_t mat) {
-    const uint32_t dx = (uint32_t)(x - lo[0]), dy = (uint32_t)(y - lo[1]), dz = (uint32_t)(z - lo[2]);
-    if (dx >= (uint32_t)kCV || dy >= (uint32_t)kCV || dz >= (uint32_t)kCV) return;
+// try_write_tree_voxel, voxel.rs:1500-1525, on the shared chunk; (x, y, z)
+// inside it
+__device__ __forceinline__ void tree_voxel(uint8_t *s_mat, uint32_t dx, uint32_t dy, uint32_t dz,
+                                           uint8_t mat) {
     const uint32_t v = vox(dx, dy, dz);
     const uint8_t cur = s_mat[v];
     if (cur == 0 || (cur == M_FRINGE && mat != M_FRINGE)) s_mat[v] = mat;
 }
 
-// Voxel k of a primitive (any order: one primitive writes one material).
-__device__ void paint_prim(uint8_t *s_mat, const int32_t lo[3], const Prim &p, int nthr) {
+// One warp paints a primitive's voxels in the slab [zlo, zhi) of the chunk at
+// lo (any order: one primitive writes one material).
+__device__ __forceinline__ void paint_prim(uint8_t *s_mat, const int32_t lo[3], int32_t zlo,
+                                           int32_t zhi, const Prim &p) {
     const uint32_t kind = p.kind_mat >> 8;
     const uint8_t mat = (uint8_t)(p.kind_mat & 0xFFu);
+    const int32_t lane = (int32_t)(threadIdx.x & 31u);
     if (kind == PR_LINE) {
-        if (p.steps <= 0) {
-            if (threadIdx.x == 0) tree_voxel(s_mat, lo, p.a[0], p.a[1], p.a[2], mat);
-            return;
-        }
         const int32_t d0 = p.b[0] - p.a[0], d1 = p.b[1] - p.a[1], d2 = p.b[2] - p.a[2];
-        for (int32_t s = (int32_t)threadIdx.x; s <= p.steps; s += nthr) {
-            const float t = (float)s / (float)p.steps;
+        const int32_t steps = max(p.steps, 0);     // no steps: the point a
+        for (int32_t s = lane; s <= steps; s += 32) {
+            const float t = steps > 0 ? (float)s / (float)steps : 0.0f;
             const int32_t x = f2i(roundf((float)p.a[0] + (float)d0 * t));
             const int32_t y = f2i(roundf((float)p.a[1] + (float)d1 * t));
             const int32_t z = f2i(roundf((float)p.a[2] + (float)d2 * t));
-            tree_voxel(s_mat, lo, x, y, z, mat);
+            if ((uint32_t)(x - lo[0]) < (uint32_t)kCV && (uint32_t)(y - lo[1]) < (uint32_t)kCV &&
+                z >= zlo && z < zhi)
+                tree_voxel(s_mat, (uint32_t)(x - lo[0]), (uint32_t)(y - lo[1]),
+                           (uint32_t)(z - lo[2]), mat);
         }
-    } else if (kind == PR_SHELL) {
-        const int32_t r = p.b[0], r2 = r * r, wxz = 2 * r + 3, n = (2 * r + 1) * wxz * wxz;
-        for (int32_t k = (int32_t)threadIdx.x; k < n; k += nthr) {
-            const int32_t dz = k % wxz - (r + 1), dx = (k / wxz) % wxz - (r + 1),
-                          dy = k / (wxz * wxz) - r;
-            const int32_t hx = max(abs(dx) - 1, 0), hz = max(abs(dz) - 1, 0);
-            if (hx * hx + dy * dy + hz * hz > r2) continue;
-            tree_voxel(s_mat, lo, p.a[0] + dx, p.a[1] + dy, p.a[2] + dz, mat);
-        }
-    } else {
-        const int32_t r = p.b[0], r2 = r * r, wd = 2 * r + 1, n = wd * wd * wd;
-        for (int32_t k = (int32_t)threadIdx.x; k < n; k += nthr) {
-            const int32_t dz = k % wd - r, dx = (k / wd) % wd - r, dy = k / (wd * wd) - r;
-            if (dx * dx + dy * dy + dz * dz > r2) continue;
-            tree_voxel(s_mat, lo, p.a[0] + dx, p.a[1] + dy, p.a[2] + dz, mat);
+        return;
+    }
+    // shell: max(|dx| - 1, 0)^2 + dy^2 + max(|dz| - 1, 0)^2 <= r^2; sphere
+    // without the widening.  Two rows of 16 voxels a round.
+    const int32_t wide = kind == PR_SHELL ? 1 : 0, r = p.b[0], r2 = r * r;
+    const int32_t ya = max(p.a[1] - r, lo[1]), yb = min(p.a[1] + r, lo[1] + kCV - 1);
+    const int32_t za = max(p.a[2] - r - wide, zlo), zb = min(p.a[2] + r + wide, zhi - 1);
+    for (int32_t z = za; z <= zb; ++z) {
+        const int32_t hz = max(abs(z - p.a[2]) - wide, 0);
+        for (int32_t y = ya + (lane >> 4); y <= yb; y += 2) {
+            const int32_t dy = y - p.a[1], rest = r2 - hz * hz - dy * dy;
+            for (int32_t dx = (lane & 15) - r - wide; dx <= r + wide; dx += 16) {
+                const int32_t hx = max(abs(dx) - wide, 0);
+                const uint32_t x = (uint32_t)(p.a[0] + dx - lo[0]);
+                if (hx * hx <= rest && x < (uint32_t)kCV)
+                    tree_voxel(s_mat, x, (uint32_t)(y - lo[1]), (uint32_t)(z - lo[2]), mat);
+            }
         }
     }
 }
@@ -408,8 +427,7 @@ __device__ __forceinline__ void src_chunk(const GenPlan &p, const Dims &d, uint3
     }
 }
 
-__global__ void __launch_bounds__(256) k_gen_columns(GenPlan p, Dims d, Seed g) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ void gen_column(const GenPlan &p, const Dims &d, const Seed &g, uint32_t c) {
     if (c >= p.n_cols * (uint32_t)(kCV * kCV)) return;
     const uint32_t k = c >> 10, col = c & 1023u;
     int32_t ccx, ccz;
@@ -456,10 +474,10 @@ __global__ void __launch_bounds__(256) k_gen_columns(GenPlan p, Dims d, Seed g) 
 }
 
 // ------------------------------------------------------------------ trees
-// Per source chunk: kCand headers (primitive count | base y << 8, 0 when the
-// candidate yields no tree) and kCand x kPrims primitives.
-__global__ void __launch_bounds__(128) k_gen_trees(GenPlan p, Dims d, Seed g) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+// Per source chunk: kCand headers (primitive count | x in the chunk << 8 |
+// z << 13 | base y << 18; 0 when the candidate yields no tree) and kCand x
+// kPrims primitives.
+__device__ void gen_tree(const GenPlan &p, const Dims &d, const Seed &g, uint32_t c) {
     if (c >= p.n_srcs * (uint32_t)kCand) return;
     const uint32_t k = c / kCand, i = c % kCand;
     int32_t scx, scz;
@@ -471,9 +489,17 @@ __global__ void __launch_bounds__(128) k_gen_trees(GenPlan p, Dims d, Seed g) {
         e.out = reinterpret_cast<Prim *>(p.prims) + (size_t)c * kPrims;
         e.n = 0;
         tree_prims(t, g.lmx, e);
-        h = e.n | (t.y << 8);
+        h = e.n | ((t.x - scx * kCV) << 8) | ((t.z - scz * kCV) << 13) | (t.y << 18);
     }
     p.hdr[c] = h;
+}
+
+// The columns and the trees in one launch: the trees are few threads with a
+// long chain of work each (35-40 us as a launch of their own), so their CTAs
+// go first and the columns' run beside them.
+__global__ void __launch_bounds__(256) k_gen_xz(GenPlan p, Dims d, Seed g, uint32_t tree_ctas) {
+    if (blockIdx.x < tree_ctas) gen_tree(p, d, g, blockIdx.x * blockDim.x + threadIdx.x);
+    else gen_column(p, d, g, (blockIdx.x - tree_ctas) * blockDim.x + threadIdx.x);
 }
 
 // ------------------------------------------------------------------ chunks
@@ -488,9 +514,10 @@ __device__ __forceinline__ void job_of(const GenPlan &p, const Dims &d, uint32_t
         for (int k = 0; k < kGenJobInts; ++k) job[k] = p.jobs[(size_t)b * kGenJobInts + k];
         return;
     }
-    const int32_t sxn = d.bx / 8, syn = d.by / 8, szn = d.bz / 8;
-    const int32_t sx = (int32_t)b % sxn, sy = ((int32_t)b / sxn) % syn,
-                  sz = (int32_t)b / (sxn * syn);
+    const int32_t sxn = d.bx / 8, szn = d.bz / 8;
+    // y slowest: the chunks below ground, which take longest, start first
+    const int32_t sx = (int32_t)b % sxn, sz = ((int32_t)b / sxn) % szn,
+                  sy = (int32_t)b / (sxn * szn);
     const int32_t cx = p.ox + wrap(sx - p.ox, sxn), cz = p.oz + wrap(sz - p.oz, szn);
     job[0] = cx; job[1] = sy; job[2] = cz;
     job[3] = sx; job[4] = sy; job[5] = sz;
@@ -500,9 +527,70 @@ __device__ __forceinline__ void job_of(const GenPlan &p, const Dims &d, uint32_t
         job[7 + k] = (cx + k % 3 - 1 - (p.ox - 1)) + (cz + k / 3 - 1 - (p.oz - 1)) * (sxn + 2);
 }
 
+// The two ore noises of stone_or_ore (voxel.rs:1906-1916) over half a chunk,
+// 16 levels at a time: the hashes of the lattice points the half can touch
+// lie in shared memory, and what depends on y alone -- the lattice row and
+// the smoothed fraction -- in a table of the chunk's 32 levels.
+// A voxel column by itself hashes each of its lattice cells' new corners (36
+// and 74 hashes per column for the two frequencies, 1,024 columns); a half
+// has 847 and 4,400 lattice points.
+constexpr float kOreF1 = 0.27f, kOreF2 = 0.55f;
+constexpr int kHalf = 16;
+constexpr int kN1 = 11, kY1 = 7, kN2 = 20, kY2 = 11;   // points: 31 f + 2 and 15 f + 2, rounded up
+struct OreLevel {
+    float yf, yg;       // smoothed fraction and 1 - it
+    int32_t yi;         // lattice row
+    int32_t pad;
+};
+struct SlotShared {
+    uint8_t mat[kCV * kCV * kCV];
+    float t1[kY1 * kN1 * kN1], t2[kY2 * kN2 * kN2];
+    OreLevel l1[kCV], l2[kCV];
+    int32_t job[kGenJobInts];
+    uint8_t uni[512], solid[512];   // per brick: uniform byte, any voxel
+};
+// one noise of a column, read from the lattice table: value_noise_3d's
+// operations on the same hashes
+template <int N>
+struct OreColumn {
+    const float *t;     // the column's lattice cell in the table, row 0
+    float xf, xg, zf, zg;
+    float a, b, c, d;
+    int32_t yi;
+    __device__ __forceinline__ float lerp(const float *q) const { return q[0] * xg + q[1] * xf; }
+    __device__ __forceinline__ float eval(const OreLevel &l, int32_t y_first) {
+        if (l.yi != yi) {
+            const float *q = t + (l.yi - y_first) * (N * N);
+            if (l.yi == yi + 1) {
+                a = b;
+                c = d;
+            } else {
+                a = lerp(q);
+                c = lerp(q + N);
+            }
+            b = lerp(q + N * N);
+            d = lerp(q + N * N + N);
+            yi = l.yi;
+        }
+        const float ab = a * l.yg + b * l.yf;
+        const float cd = c * l.yg + d * l.yf;
+        return ab * zg + cd * zf;
+    }
+};
+__device__ __forceinline__ uint8_t ore_of(float n1, float n2, int32_t depth) {
+    const float combined = n1 + n2 * 0.30f;
+    if (depth > 30 && combined > 0.50f) return M_DIAMOND;
+    if (depth > 20 && combined > 0.36f) return M_GOLD;
+    if (depth > 10 && combined > 0.24f) return M_IRON;
+    if (combined > 0.32f) return M_COAL;
+    return M_STONE;
+}
+
 __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPlan pl) {
-    __shared__ __align__(16) uint8_t s_mat[kCV * kCV * kCV];
-    __shared__ int32_t s_job[kGenJobInts];
+    extern __shared__ __align__(16) uint8_t s_raw[];
+    SlotShared &sh = *reinterpret_cast<SlotShared *>(s_raw);
+    uint8_t *s_mat = sh.mat;
+    int32_t *s_job = sh.job;
     if (threadIdx.x == 0) {
         int32_t j[kGenJobInts];
         job_of(pl, w.d, blockIdx.x, j);
@@ -521,59 +609,121 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
     const uint32_t *colw = pl.colw + (size_t)job[6] * (kCV * kCV);
 
     // ---- the columns (dx, dz), voxel.rs:1333-1461
+    // Thread: dx = its lane, dz = its warp + 8 i.
     const int32_t y0 = lo[1];
-    for (uint32_t col = tid; col < (uint32_t)(kCV * kCV); col += kSlotThreads) {
-        const uint32_t word = colw[col];
-        const int32_t h = (int32_t)(word & 0xFFu);
-        const uint32_t hu = (uint32_t)h;
-        const int32_t water_top = (word >> 8) & 1u ? kSea : 0;
-        const int col_top = max(h, water_top);
-        if (col_top < y0 || 0 >= y0 + kCV) continue;
-        const int biome = (int)((word >> 9) & 7u);
-        const uint32_t dx = col & 31u, dz = col >> 5;
-        const float wx = (float)(lo[0] + (int32_t)dx), wz = (float)(lo[2] + (int32_t)dz);
-        const int32_t ys = max(y0, 0), ye = min(y0 + kCV, kWorldY);
-        const int32_t seal = water_top > h ? h - 5 : INT32_MIN;
-        // stone_or_ore's two noises (voxel.rs:1906-1916) along this column
-        // and the two cave noises (:1361-1366)
-        noise::ColumnNoise3 ore1, ore2, cave1, cave2;
-        ore1.init(wx * 0.27f, wz * 0.27f);
-        ore2.init(wx * 0.55f, wz * 0.55f);
-        cave1.init(wx * 0.045f, wz * 0.045f);
-        cave2.init(wx * 0.110f, wz * 0.110f);
-        for (int32_t y = ys; y < ye; ++y) {
-            if (y > h) break;
-            if (!(y >= seal) && y > 4 && y + 3 < h) {
-                const float cn = cave1.eval((float)y * 0.085f);
-                const float cn2 = cave2.eval((float)y * 0.060f);
-                if ((cn + cn2 * 0.6f) > 0.30f) continue;
-            }
-            uint8_t mat;
-            if ((uint32_t)y >= hu) {
-                mat = top_block(biome, hu);
-            } else if ((uint32_t)y + 4u >= hu) {
-                mat = subsoil(biome);
-            } else {
-                const float fy = (float)y;
-                const float depth = fmaxr((float)hu - fy, 0.0f);
-                const float n1 = ore1.eval(fy * 0.27f);
-                const float n2 = ore2.eval(fy * 0.55f);
-                const float combined = n1 + n2 * 0.30f;
-                if (depth > 30.0f && combined > 0.50f) mat = M_DIAMOND;
-                else if (depth > 20.0f && combined > 0.36f) mat = M_GOLD;
-                else if (depth > 10.0f && combined > 0.24f) mat = M_IRON;
-                else if (combined > 0.32f) mat = M_COAL;
-                else mat = M_STONE;
-            }
-            s_mat[vox(dx, (uint32_t)(y - y0), dz)] = mat;
+    const uint32_t lane = tid & 31u, warp = tid >> 5;
+    const int32_t wxi = lo[0] + (int32_t)lane;
+    const float wx = (float)wxi;
+    // x and z lattice cells; a chunk so far out that binary32 coordinates
+    // skip cells does not fit the tables and evaluates its noise directly
+    const int32_t x1 = noise::floor_i((float)lo[0] * kOreF1), x2 = noise::floor_i((float)lo[0] * kOreF2);
+    const int32_t z1 = noise::floor_i((float)lo[2] * kOreF1), z2 = noise::floor_i((float)lo[2] * kOreF2);
+    const float xe = (float)(lo[0] + kCV - 1), ze = (float)(lo[2] + kCV - 1);
+    const bool tables = noise::floor_i(xe * kOreF1) - x1 + 2 <= kN1 &&
+                        noise::floor_i(ze * kOreF1) - z1 + 2 <= kN1 &&
+                        noise::floor_i(xe * kOreF2) - x2 + 2 <= kN2 &&
+                        noise::floor_i(ze * kOreF2) - z2 + 2 <= kN2;
+    if (tid < (uint32_t)kCV) {
+        const float fy = (float)(y0 + (int32_t)tid);
+        const float p1 = fy * kOreF1, p2 = fy * kOreF2;
+        const int32_t i1 = noise::floor_i(p1), i2 = noise::floor_i(p2);
+        const float f1 = noise::smooth(p1 - (float)i1), f2 = noise::smooth(p2 - (float)i2);
+        sh.l1[tid] = OreLevel{f1, 1.0f - f1, i1, 0};
+        sh.l2[tid] = OreLevel{f2, 1.0f - f2, i2, 0};
+    }
+    uint32_t words[4];
+    int32_t h_max = -1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        words[i] = colw[tid + (uint32_t)(kSlotThreads * i)];
+        h_max = max(h_max, (int32_t)(words[i] & 0xFFu));
+    }
+    for (int half = 0; half < kCV / kHalf; ++half) {
+        const int32_t ylo = y0 + half * kHalf, yhi = ylo + kHalf;
+        // any voxel of stone or ore (y + 4 < h) in this half?
+        const bool ore = __syncthreads_or(ylo + 4 < h_max) != 0 && tables;
+        const int32_t r1 = sh.l1[half * kHalf].yi, r2 = sh.l2[half * kHalf].yi;
+        if (ore) {
+            for (uint32_t i = tid; i < (uint32_t)(kY1 * kN1 * kN1); i += kSlotThreads)
+                sh.t1[i] = hash3(x1 + (int32_t)(i % kN1), r1 + (int32_t)(i / (kN1 * kN1)),
+                                 z1 + (int32_t)((i / kN1) % kN1));
+            for (uint32_t i = tid; i < (uint32_t)(kY2 * kN2 * kN2); i += kSlotThreads)
+                sh.t2[i] = hash3(x2 + (int32_t)(i % kN2), r2 + (int32_t)(i / (kN2 * kN2)),
+                                 z2 + (int32_t)((i / kN2) % kN2));
+            __syncthreads();
         }
-        if (water_top > h) {
-            const int32_t fb = max(h + 1, y0), fe = min(water_top, y0 + kCV - 1);
-            for (int32_t wy = fb; wy <= fe; ++wy) s_mat[vox(dx, (uint32_t)(wy - y0), dz)] = M_WATER;
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t word = words[i];
+            const int32_t h = (int32_t)(word & 0xFFu);
+            const uint32_t hu = (uint32_t)h;
+            const int32_t water_top = (word >> 8) & 1u ? kSea : 0;
+            const int col_top = max(h, water_top);
+            if (col_top < ylo) continue;
+            const int biome = (int)((word >> 9) & 7u);
+            const uint32_t dx = lane, dz = warp + 8u * (uint32_t)i;
+            const float wz = (float)(lo[2] + (int32_t)dz);
+            const int32_t ye = min(yhi, kWorldY);
+            int32_t y = ylo;
+            // below the subsoil, caves only under water (their seal): stone and ore
+            const int32_t seal = water_top > h ? h - 5 : INT32_MIN;
+            const int32_t ore_end = min(ye, h - 4);      // y + 4 < h
+            if (ore && seal == INT32_MIN) {
+                OreColumn<kN1> o1;
+                OreColumn<kN2> o2;
+                const float px1 = wx * kOreF1, pz1 = wz * kOreF1, px2 = wx * kOreF2, pz2 = wz * kOreF2;
+                const int32_t xi1 = noise::floor_i(px1), zi1 = noise::floor_i(pz1);
+                const int32_t xi2 = noise::floor_i(px2), zi2 = noise::floor_i(pz2);
+                o1.xf = noise::smooth(px1 - (float)xi1); o1.xg = 1.0f - o1.xf;
+                o1.zf = noise::smooth(pz1 - (float)zi1); o1.zg = 1.0f - o1.zf;
+                o2.xf = noise::smooth(px2 - (float)xi2); o2.xg = 1.0f - o2.xf;
+                o2.zf = noise::smooth(pz2 - (float)zi2); o2.zg = 1.0f - o2.zf;
+                o1.t = sh.t1 + (zi1 - z1) * kN1 + (xi1 - x1);
+                o2.t = sh.t2 + (zi2 - z2) * kN2 + (xi2 - x2);
+                o1.yi = o2.yi = INT32_MIN;
+                for (; y < ore_end; ++y) {
+                    const float n1 = o1.eval(sh.l1[y - y0], r1);
+                    const float n2 = o2.eval(sh.l2[y - y0], r2);
+                    s_mat[vox(dx, (uint32_t)(y - y0), dz)] = ore_of(n1, n2, h - y);
+                }
+            }
+            if (y < ye && y <= h) {
+                // the rest of the column: surface and subsoil, and whole
+                // columns with caves or beyond the tables
+                noise::ColumnNoise3 ore1, ore2, cave1, cave2;
+                ore1.init(wx * kOreF1, wz * kOreF1);
+                ore2.init(wx * kOreF2, wz * kOreF2);
+                cave1.init(wx * 0.045f, wz * 0.045f);
+                cave2.init(wx * 0.110f, wz * 0.110f);
+                for (; y < ye; ++y) {
+                    if (y > h) break;
+                    if (!(y >= seal) && y > 4 && y + 3 < h) {
+                        const float cn = cave1.eval((float)y * 0.085f);
+                        const float cn2 = cave2.eval((float)y * 0.060f);
+                        if ((cn + cn2 * 0.6f) > 0.30f) continue;
+                    }
+                    uint8_t mat;
+                    if ((uint32_t)y >= hu) mat = top_block(biome, hu);
+                    else if ((uint32_t)y + 4u >= hu) mat = subsoil(biome);
+                    else mat = ore_of(ore1.eval((float)y * kOreF1), ore2.eval((float)y * kOreF2), h - y);
+                    s_mat[vox(dx, (uint32_t)(y - y0), dz)] = mat;
+                }
+            }
+            if (water_top > h) {
+                const int32_t fb = max(h + 1, ylo), fe = min(water_top, yhi - 1);
+                for (int32_t wy = fb; wy <= fe; ++wy)
+                    s_mat[vox(dx, (uint32_t)(wy - y0), dz)] = M_WATER;
+            }
         }
-        const uint32_t dec = (word >> 12) & 63u;
-        const int32_t dec_y = h + 1;
-        if (dec != 0u && dec_y >= y0 && dec_y < y0 + kCV) {
+        __syncthreads();                 // before the tables change
+    }
+    // surface decoration over the finished columns
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t word = words[i];
+        const uint32_t dec = (word >> 12) & 63u, dx = lane, dz = warp + 8u * (uint32_t)i;
+        const int32_t dec_y = (int32_t)(word & 0xFFu) + 1;
+        // a column that ends below the chunk decorates nothing in it
+        if (dec != 0u && dec_y > y0 && dec_y < y0 + kCV) {
             const uint32_t dy = (uint32_t)(dec_y - y0);
             s_mat[vox(dx, dy, dz)] = (uint8_t)dec;
             if (((word >> 18) & 1u) && dec_y + 1 < y0 + kCV) s_mat[vox(dx, dy + 1u, dz)] = M_BUSH;
@@ -581,23 +731,65 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
     }
     __syncthreads();
 
-    // ---- trees of the 3x3 source chunks in the reference's order
-    for (int k = 0; k < 9; ++k) {
-        const int32_t src = job[7 + k];
-        for (int i = 0; i < kCand; ++i) {
-            const int32_t hd = pl.hdr[(size_t)src * kCand + i];
-            const int np = hd & 0xFF;
-            const int32_t base_y = hd >> 8;
-            if (np == 0 || base_y > lo[1] + kCV || base_y + 22 < lo[1]) continue;
-            const Prim *tp = prims + ((size_t)src * kCand + i) * kPrims;
-            for (int p = 0; p < np; ++p) {
-                const Prim pr = tp[p];
-                if (!prim_meets(pr, lo)) continue;
-                paint_prim(s_mat, lo, pr, kSlotThreads);
-                __syncthreads();
+    // ---- trees of the 3x3 source chunks in the reference's order, a slab of
+    // four z levels per warp: the warp takes every primitive that can reach
+    // its slab, in order, so no other thread writes its voxels
+    {
+        const int32_t zlo = lo[2] + 4 * (int32_t)warp, zhi = zlo + 4;
+        int32_t hd[(kTrees + 31) / 32];
+#pragma unroll
+        for (int q = 0; q < (kTrees + 31) / 32; ++q) {
+            const int c = q * 32 + (int)lane;
+            hd[q] = 0;
+            if (c < kTrees) hd[q] = __ldg(pl.hdr + (size_t)job[7 + c / kCand] * kCand + c % kCand);
+        }
+#pragma unroll
+        for (int q = 0; q < (kTrees + 31) / 32; ++q) {
+            const int c = q * 32 + (int)lane, k = c / kCand;
+            const int32_t bx = (job[0] + k % 3 - 1) * kCV + ((hd[q] >> 8) & 31);
+            const int32_t bz = (job[2] + k / 3 - 1) * kCV + ((hd[q] >> 13) & 31);
+            const int32_t by = hd[q] >> 18;
+            uint32_t near = __ballot_sync(
+                0xFFFFFFFFu, (hd[q] & 0xFF) != 0 && by <= lo[1] + kCV && by + 22 >= lo[1] &&
+                                 bx + kTreeReach >= lo[0] && bx - kTreeReach < lo[0] + kCV &&
+                                 bz + kTreeReach >= zlo && bz - kTreeReach < zhi);
+            while (near != 0u) {
+                const int l = __ffs((int)near) - 1;
+                near &= near - 1u;
+                const int tc = q * 32 + l, np = __shfl_sync(0xFFFFFFFFu, hd[q], l) & 0xFF;
+                // one primitive per lane; those that reach the slab, in order
+                Prim mine{};
+                bool meets = false;
+                if ((int)lane < np) {
+                    const Prim *tp = prims + ((size_t)job[7 + tc / kCand] * kCand + tc % kCand) * kPrims;
+                    const int4 a = __ldg(reinterpret_cast<const int4 *>(tp + lane));
+                    const int4 b = __ldg(reinterpret_cast<const int4 *>(tp + lane) + 1);
+                    mine.a[0] = a.x; mine.a[1] = a.y; mine.a[2] = a.z; mine.b[0] = a.w;
+                    mine.b[1] = b.x; mine.b[2] = b.y; mine.kind_mat = (uint32_t)b.z; mine.steps = b.w;
+                    int32_t mn[3], mx[3];
+                    prim_box(mine, mn, mx);
+                    meets = mx[0] >= lo[0] && mn[0] < lo[0] + kCV && mx[1] >= lo[1] &&
+                            mn[1] < lo[1] + kCV && mx[2] >= zlo && mn[2] < zhi;
+                }
+                uint32_t todo = __ballot_sync(0xFFFFFFFFu, meets);
+                while (todo != 0u) {
+                    const int o = __ffs((int)todo) - 1;
+                    todo &= todo - 1u;
+                    Prim pr;
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) {
+                        pr.a[m] = __shfl_sync(0xFFFFFFFFu, mine.a[m], o);
+                        pr.b[m] = __shfl_sync(0xFFFFFFFFu, mine.b[m], o);
+                    }
+                    pr.kind_mat = __shfl_sync(0xFFFFFFFFu, mine.kind_mat, o);
+                    pr.steps = __shfl_sync(0xFFFFFFFFu, mine.steps, o);
+                    paint_prim(s_mat, lo, zlo, zhi, pr);
+                    __syncwarp();
+                }
             }
         }
     }
+    __syncthreads();
 
     // ---- bricks out: material rows, occupancy words, uniform bytes
     const uint32_t sbx = (uint32_t)job[3] * 8u, sby = (uint32_t)job[4] * 8u,
@@ -624,7 +816,36 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
             }
         }
         w.occ[gbi] = occ;
-        w.brick_uniform[gbi] = (occ == ~0ull && same) ? (uint8_t)m0 : (uint8_t)0;
+        const uint8_t u = (occ == ~0ull && same) ? (uint8_t)m0 : (uint8_t)0;
+        w.brick_uniform[gbi] = u;
+        sh.uni[b] = u;
+        sh.solid[b] = occ != 0ull ? 1u : 0u;
+    }
+    __syncthreads();
+    // the chunk's eight tiles, one warp each (tile word and LUT,
+    // voxel.rs:253-272, :964-972): their bricks are all here
+    {
+        const uint32_t tx = warp & 1u, ty = (warp >> 1) & 1u, tz = warp >> 2;
+        uint32_t u[2], sol[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const uint32_t c = lane + 32u * (uint32_t)q;   // child bit x + z*4 + y*16
+            const uint32_t b = (tx * 4u + (c & 3u)) + (ty * 4u + (c >> 4)) * 8u +
+                               (tz * 4u + ((c >> 2) & 3u)) * 64u;
+            u[q] = sh.uni[b];
+            sol[q] = sh.solid[b];
+        }
+        const uint32_t m_lo = __ballot_sync(0xFFFFFFFFu, sol[0] != 0u);
+        const uint32_t m_hi = __ballot_sync(0xFFFFFFFFu, sol[1] != 0u);
+        const uint32_t m0 = __shfl_sync(0xFFFFFFFFu, u[0], 0);
+        const bool uni = __all_sync(0xFFFFFFFFu, m0 != 0u && u[0] == m0 && u[1] == m0);
+        if (lane == 0u) {
+            const int64_t ti = (int64_t)(job[3] * 2 + (int32_t)tx) +
+                               (int64_t)(job[4] * 2 + (int32_t)ty) * w.d.tx +
+                               (int64_t)(job[5] * 2 + (int32_t)tz) * w.d.tx * w.d.ty;
+            w.tile_mask[ti] = (uint64_t)m_lo | ((uint64_t)m_hi << 32);
+            w.tile_uniform[ti] = uni ? (uint8_t)m0 : (uint8_t)0;
+        }
     }
 }
 
@@ -654,7 +875,8 @@ cudaError_t launch_gen_math(const uint32_t *lmx, uint32_t fn, const float *in, s
 
 size_t gen_prim_bytes_per_src() { return sizeof(Prim) * kCand * kPrims; }
 
-cudaError_t launch_gen_slots(const DevWorld &w, uint64_t seed, const GenPlan &p, cudaStream_t s) {
+cudaError_t launch_gen_slots(const DevWorld &w, uint64_t seed, const GenPlan &p, bool tiles_built,
+                             cudaStream_t s) {
     if (p.n_jobs == 0) return cudaSuccess;
     Seed g;
     g.seed = seed;
@@ -663,14 +885,16 @@ cudaError_t launch_gen_slots(const DevWorld &w, uint64_t seed, const GenPlan &p,
     g.offz = (float)(int32_t)(uint32_t)(seed & 0xFFFFFFFFull) * 0.02153f;
     g.lmx = p.lmx;
     if (!g.lmx) return cudaErrorInvalidValue;
-    const uint32_t n_col_threads = p.n_cols * (uint32_t)(kCV * kCV);
-    k_gen_columns<<<(n_col_threads + 255) / 256, 256, 0, s>>>(p, w.d, g);
-    const uint32_t n_tree_threads = p.n_srcs * (uint32_t)kCand;
-    k_gen_trees<<<(n_tree_threads + 127) / 128, 128, 0, s>>>(p, w.d, g);
-    k_gen_slot<<<p.n_jobs, kSlotThreads, 0, s>>>(w, p);
-    cudaError_t e = cudaGetLastError();
+    const uint32_t col_ctas = (p.n_cols * (uint32_t)(kCV * kCV) + 255u) / 256u;
+    const uint32_t tree_ctas = (p.n_srcs * (uint32_t)kCand + 255u) / 256u;
+    k_gen_xz<<<tree_ctas + col_ctas, 256, 0, s>>>(p, w.d, g, tree_ctas);
+    cudaError_t e = cudaFuncSetAttribute(k_gen_slot, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(SlotShared));
     if (e != cudaSuccess) return e;
-    return launch_rebuild_pyramid(w, s);
+    k_gen_slot<<<p.n_jobs, kSlotThreads, sizeof(SlotShared), s>>>(w, p);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return launch_rebuild_pyramid(w, !tiles_built, s);
 }
 
 }  // namespace vx

@@ -430,12 +430,12 @@ cudaError_t launch_bricks_to_aos(const DevWorld &w, VxBrick *aos, int64_t first,
     return cudaGetLastError();
 }
 
-cudaError_t launch_rebuild_pyramid(const DevWorld &w, cudaStream_t s) {
+cudaError_t launch_rebuild_pyramid(const DevWorld &w, bool tiles, cudaStream_t s) {
     // one thread per tile needs enough tiles to hide its chain of loads
     // (16,384 tiles: 17 us against 8 us for a warp each)
-    if (w.d.n_tiles > 65536)
+    if (tiles && w.d.n_tiles > 65536)
         k_build_tiles_stream<<<blocks_for(w.d.n_tiles, 128), 128, 0, s>>>(w);
-    else
+    else if (tiles)
         k_build_tiles<<<warp_blocks(w.d.n_tiles), 256, 0, s>>>(w);
     k_build_chunks<<<warp_blocks(w.d.n_chunks), 256, 0, s>>>(w);
     k_build_l4<<<warp_blocks(w.d.n_l4), 256, 0, s>>>(w);
@@ -457,7 +457,7 @@ cudaError_t launch_generate(const DevWorld &w, const VxTerrainParams &t, int16_t
     g.heights = heights;
     k_heights<<<blocks_for((int64_t)w.d.vx * w.d.vz, 256), 256, 0, s>>>(g);
     k_gen_bricks<<<blocks_for(w.d.n_bricks, 128), 128, 0, s>>>(g);
-    return launch_rebuild_pyramid(w, s);
+    return launch_rebuild_pyramid(w, true, s);
 }
 
 // win: a claim word per brick, zero between updates (the last of an update's
