@@ -29,6 +29,7 @@ namespace vx {
 namespace {
 
 constexpr uint32_t kTileItems = 2048;   // radix sort: items per warp-tile
+constexpr uint32_t kPasses = 4;         // 8-bit digits of the key
 
 struct QueueArgs {
     TraceArgs ta;
@@ -48,6 +49,33 @@ __device__ __forceinline__ void load_ray(const VxRay *rays, uint32_t i, float &o
     const float4 b = __ldg(reinterpret_cast<const float4 *>(rays + i) + 1);
     ox = a.x; oy = a.y; oz = a.z; dx = a.w; dy = b.x; dz = b.y; tmax = b.z;
     kind = __float_as_uint(b.w);
+}
+
+// The shadow ray of ray `ray` after its hit h (raymarch.wgsl:3953-3994: the
+// origin p_hit + n*0.001, the sun direction jittered in its cone); the jitter
+// is seeded by the ray index.
+struct ShadowRay {
+    float ox, oy, oz, dx, dy, dz;
+};
+__device__ __forceinline__ ShadowRay shadow_of(const VxTraceParams &p, uint32_t ray, float ox,
+                                               float oy, float oz, float dx, float dy, float dz,
+                                               const Hit &h) {
+    ShadowRay r;
+    const int ax = (int)(h.face >> 1);
+    const float nv = (h.face & 1u) ? -1.0f : 1.0f;
+    r.ox = (ox + dx * h.t) + (ax == 0 ? nv : 0.0f) * 0.001f;
+    r.oy = (oy + dy * h.t) + (ax == 1 ? nv : 0.0f) * 0.001f;
+    r.oz = (oz + dz * h.t) + (ax == 2 ? nv : 0.0f) * 0.001f;
+    const float jit = ign((float)(ray & 0xFFFFu), (float)(ray >> 16), p.frame);
+    const float theta = jit * 2.39996323f;
+    const float radius = p.cone_tan * sqrtf(jit);
+    float sn, cs;
+    sincos_series(theta, sn, cs);
+    r.dx = p.sun[0] + (p.sun_tangent[0] * cs + p.sun_bitangent[0] * sn) * radius;
+    r.dy = p.sun[1] + (p.sun_tangent[1] * cs + p.sun_bitangent[1] * sn) * radius;
+    r.dz = p.sun[2] + (p.sun_tangent[2] * cs + p.sun_bitangent[2] * sn) * radius;
+    normalize3(r.dx, r.dy, r.dz);
+    return r;
 }
 
 template <uint32_t FL>
@@ -114,35 +142,85 @@ __global__ void __launch_bounds__(256) k_queue(QueueArgs q) {
                     h.steps = k.iters;
                     store_record(q.out + ray, h);
                     if (q.shadow && (rkind & VX_RAY_SPAWN_SHADOW) && r == WALK_HIT) {
-                        {
-                            // raymarch.wgsl:3953-3994 from this ray's hit; the
-                            // jitter is seeded by the ray index
-                            const int ax = (int)(h.face >> 1);
-                            const float nv = (h.face & 1u) ? -1.0f : 1.0f;
-                            const float sox = (ox + k.s.dx * h.t) + (ax == 0 ? nv : 0.0f) * 0.001f;
-                            const float soy = (oy + k.s.dy * h.t) + (ax == 1 ? nv : 0.0f) * 0.001f;
-                            const float soz = (oz + k.s.dz * h.t) + (ax == 2 ? nv : 0.0f) * 0.001f;
-                            const float jit = ign((float)(ray & 0xFFFFu), (float)(ray >> 16), p.frame);
-                            const float theta = jit * 2.39996323f;
-                            const float radius = p.cone_tan * sqrtf(jit);
-                            float sn, cs;
-                            sincos_series(theta, sn, cs);
-                            float sdx = p.sun[0] + (p.sun_tangent[0] * cs + p.sun_bitangent[0] * sn) * radius;
-                            float sdy = p.sun[1] + (p.sun_tangent[1] * cs + p.sun_bitangent[1] * sn) * radius;
-                            float sdz = p.sun[2] + (p.sun_tangent[2] * cs + p.sun_bitangent[2] * sn) * radius;
-                            normalize3(sdx, sdy, sdz);
-                            if (walk_init(w.d, ro, KIND_ANY, p, sox, soy, soz, sdx, sdy, sdz,
-                                          p.shadow_max_dist, k)) {
-                                shadow_phase = true;
-                                item = 0u;
-                            } else {
-                                reinterpret_cast<uint2 *>(q.shadow)[ray] = make_uint2(0u, 1u << 8);
-                            }
+                        const ShadowRay sr =
+                            shadow_of(p, ray, ox, oy, oz, k.s.dx, k.s.dy, k.s.dz, h);
+                        if (walk_init(w.d, ro, KIND_ANY, p, sr.ox, sr.oy, sr.oz, sr.dx, sr.dy,
+                                      sr.dz, p.shadow_max_dist, k)) {
+                            shadow_phase = true;
+                            item = 0u;
+                        } else {
+                            reinterpret_cast<uint2 *>(q.shadow)[ray] = make_uint2(0u, 1u << 8);
                         }
                     }
                 }
             }
         }
+    }
+    if (lane == 0) {
+        const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+        if (atomicAdd(q.work + 1, 1u) == warps - 1u) {
+            q.work[0] = 0u;
+            q.work[1] = 0u;
+        }
+    }
+}
+
+// Whole packets (refill_min 32: a warp refills when every lane is idle): a
+// warp takes 32 queue items, walks their rays to the end, then their shadow
+// rays.  No lane changes the kind of its ray inside a walk, so the walks are
+// the kind's own, without the per-iteration votes and the kind tests of
+// k_queue, whose lanes may hold any mix.  The next packet's number is asked
+// for while the current one is walked.
+// Sorted 1080p mix (3.0M rays, 1.3M shadow rays): 632 us and 531 M warp
+// instructions as lane refill at 32, 555 us and 422 M here.  At least 3 CTAs
+// of 256 (62 registers): 2, 4 and 5 measured 3, 0.5 and 2 % slower.
+template <uint32_t FL>
+__global__ void __launch_bounds__(256, 3) k_queue_packet(QueueArgs q) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31u;
+    const DevWorld &w = q.ta.w;
+    const Ro ro{q.ta.ro[0], q.ta.ro[1], q.ta.ro[2]};
+    const VxTraceParams &p = q.ta.p;
+    uint64_t bytes = 0;
+    uint32_t next = 0;
+    if (lane == 0) next = atomicAdd(q.work, 32u);
+    for (;;) {
+        const uint32_t base = __shfl_sync(FULL, next, 0);
+        if (base >= q.n) break;
+        if (lane == 0) next = atomicAdd(q.work, 32u);
+        const uint32_t slot = base + lane;
+        if (slot < q.n) {
+            const uint32_t ray = q.order ? __ldg(q.order + slot).y : slot;
+            float ox, oy, oz, dx, dy, dz, tmax;
+            uint32_t rkind;
+            load_ray(q.rays, ray, ox, oy, oz, dx, dy, dz, tmax, rkind);
+            const uint32_t kind = rkind & 3u;
+            Hit h;
+            uint32_t ssteps = 0, sword = 0;
+            if (kind == KIND_ANY) {
+                uint32_t steps;
+                const bool occ = trace_any_ray<FL, false>(w, p, ro, ox, oy, oz, dx, dy, dz, tmax,
+                                                          steps, bytes);
+                set_miss(h);
+                h.flags = occ ? 1u : 0u;
+                h.steps = steps;
+            } else {
+                if (kind == KIND_NO_WATER)
+                    trace_no_water_ray<FL, false>(w, p, ro, ox, oy, oz, dx, dy, dz, tmax, h, bytes);
+                else
+                    trace_ray<FL, false>(w, p, ro, ox, oy, oz, dx, dy, dz, tmax, h, bytes);
+                if (q.shadow && (rkind & VX_RAY_SPAWN_SHADOW) && (h.flags & 1u)) {
+                    const ShadowRay sr = shadow_of(p, ray, ox, oy, oz, dx, dy, dz, h);
+                    const bool occ = trace_any_ray<FL, false>(w, p, ro, sr.ox, sr.oy, sr.oz, sr.dx,
+                                                              sr.dy, sr.dz, p.shadow_max_dist,
+                                                              ssteps, bytes);
+                    sword = (occ ? 1u : 0u) | (1u << 8);
+                }
+            }
+            store_record(q.out + ray, h);
+            if (q.shadow) reinterpret_cast<uint2 *>(q.shadow)[ray] = make_uint2(ssteps, sword);
+        }
+        __syncwarp();
     }
     if (lane == 0) {
         const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -166,10 +244,8 @@ __device__ __forceinline__ uint32_t spread_bits(uint32_t x) {   // 10 bits -> ev
     return x;
 }
 
-__global__ void k_radix_keys(const VxRay *rays, uint32_t n, int32_t rox, int32_t roz,
-                             uint2 *kv) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__device__ __forceinline__ uint32_t ray_key(const VxRay *rays, uint32_t i, int32_t rox,
+                                            int32_t roz) {
     float ox, oy, oz, dx, dy, dz, tmax;
     uint32_t kind;
     load_ray(rays, i, ox, oy, oz, dx, dy, dz, tmax, kind);
@@ -191,13 +267,39 @@ __global__ void k_radix_keys(const VxRay *rays, uint32_t n, int32_t rox, int32_t
         return ((uint32_t)c >> 6) & 15u;
     };
     const uint32_t oc = cell(ox, rox) | (cell(oz, roz) << 4) | ((cell(oy, 0) & 3u) << 8);
-    kv[i] = make_uint2(((kind & 3u) << 30) | (morton << 10) | oc, i);
+    return ((kind & 3u) << 30) | (morton << 10) | oc;
+}
+
+// (key, ray) pairs of a 2048-ray tile per CTA, and the tile's counts of the
+// first digit on the way (k_radix_hist counts the others').  All counts also
+// go to the digit's total over the tiles, from which k_radix_rowscan forms its
+// base: a launch per pass that summed the rows, and a first k_radix_hist, went
+// (24 us of the 1080p mix).
+// Shorter keys were no gain: 24 bits save a pass (about 45 us) and cost 75-90
+// in the walks, whose rays sort less well; 22 or 24 direction bits change
+// nothing.
+__global__ void __launch_bounds__(256) k_radix_keys(const VxRay *rays, uint32_t n, int32_t rox,
+                                                    int32_t roz, uint2 *kv, uint32_t tiles,
+                                                    uint32_t *counts, uint32_t *totals) {
+    __shared__ uint32_t h[256];
+    h[threadIdx.x] = 0u;
+    __syncthreads();
+    const uint32_t begin = blockIdx.x * kTileItems, end = min(n, begin + kTileItems);
+    for (uint32_t i = begin + threadIdx.x; i < end; i += 256u) {
+        const uint32_t key = ray_key(rays, i, rox, roz);
+        kv[i] = make_uint2(key, i);
+        atomicAdd(&h[key & 255u], 1u);
+    }
+    __syncthreads();
+    const uint32_t t = h[threadIdx.x];
+    counts[threadIdx.x * tiles + blockIdx.x] = t;
+    if (t != 0u) atomicAdd(totals + threadIdx.x, t);
 }
 
 // Per warp-tile histogram of one 8-bit digit: counts[digit * tiles + tile].
 __global__ void __launch_bounds__(128) k_radix_hist(const uint2 *kv, uint32_t n,
                                                     uint32_t shift, uint32_t tiles,
-                                                    uint32_t *counts) {
+                                                    uint32_t *counts, uint32_t *totals) {
     __shared__ uint32_t h[4][256];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     for (uint32_t d = lane; d < 256u; d += 32u) h[warp][d] = 0u;
@@ -210,11 +312,16 @@ __global__ void __launch_bounds__(128) k_radix_hist(const uint2 *kv, uint32_t n,
         __syncwarp();
         for (uint32_t d = lane; d < 256u; d += 32u) counts[d * tiles + tile] = h[warp][d];
     }
+    __syncthreads();
+    for (uint32_t d = threadIdx.x; d < 256u; d += blockDim.x) {
+        const uint32_t t = (h[0][d] + h[1][d]) + (h[2][d] + h[3][d]);
+        if (t != 0u) atomicAdd(totals + d, t);
+    }
 }
 
-// Exclusive scan of the digit-major counts: first the row totals, then each
-// row scanned by one 256-thread CTA from its digit's base (the totals of the
-// smaller digits), 1024 entries a round, four per thread.
+// Exclusive scan of the digit-major counts: each row by one 256-thread CTA
+// from its digit's base (the totals of the smaller digits), 1024 entries a
+// round, four per thread.
 __device__ __forceinline__ uint32_t block_sum256(uint32_t v, uint32_t *wsum) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -228,25 +335,12 @@ __device__ __forceinline__ uint32_t block_sum256(uint32_t v, uint32_t *wsum) {
     return t;
 }
 
-// row totals: one warp per digit row (its loads are independent, so one warp
-// keeps many in flight; a CTA per row measured slower)
-__global__ void __launch_bounds__(256) k_radix_rowsum(const uint32_t *counts, uint32_t tiles,
-                                                      uint32_t *rowsum) {
-    const uint32_t d = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-    const uint32_t *row = counts + (size_t)d * tiles;
-    uint32_t sum = 0;
-    for (uint32_t t = lane; t < tiles; t += 32u) sum += row[t];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-    if (lane == 0) rowsum[d] = sum;
-}
-
 __global__ void __launch_bounds__(256) k_radix_rowscan(uint32_t *counts, uint32_t tiles,
-                                                       const uint32_t *rowsum) {
+                                                       const uint32_t *totals) {
     __shared__ uint32_t wsum[8];
     const uint32_t d = blockIdx.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     uint32_t base = 0;
-    for (uint32_t k = tid; k < d; k += blockDim.x) base += rowsum[k];
+    for (uint32_t k = tid; k < d; k += blockDim.x) base += totals[k];
     base = block_sum256(base, wsum);
     uint32_t *row = counts + (size_t)d * tiles;
     for (uint32_t c0 = 0; c0 < tiles; c0 += 1024u) {
@@ -302,7 +396,7 @@ constexpr uint32_t kScatterWarps = 8;
 constexpr uint32_t kSliceItems = kTileItems / kScatterWarps;   // 256 = 8 rounds of 32
 __global__ void __launch_bounds__(32 * kScatterWarps) k_radix_scatter(
     const uint2 *in, uint32_t n, uint32_t shift, uint32_t tiles, const uint32_t *counts,
-    uint2 *out) {
+    uint32_t *totals, uint2 *out) {
     __shared__ __align__(16) uint2 st[kTileItems];
     __shared__ uint32_t wrank[kScatterWarps][256];   // per warp and digit: count, then first rank
     __shared__ uint32_t dfirst[256];                 // first slot of each digit in the tile
@@ -312,6 +406,7 @@ __global__ void __launch_bounds__(32 * kScatterWarps) k_radix_scatter(
     const uint32_t tile = blockIdx.x;
     const uint32_t begin = tile * kTileItems, end = min(n, begin + kTileItems);
     const uint32_t cnt = end - begin;
+    if (tile == 0u) totals[tid] = 0u;    // consumed by the row scan; zero for the next sort
     for (uint32_t i = tid; i < kScatterWarps * 256u; i += blockDim.x) (&wrank[0][0])[i] = 0u;
     __syncthreads();
     // 1. rank within the warp's slice
@@ -397,7 +492,14 @@ struct QueueK {
     static void *fn() { return reinterpret_cast<void *>(&k_queue<FL>); }
 };
 
-void *queue_kernel(uint32_t fl) { return pick_fl<QueueK>(fl); }
+template <uint32_t FL>
+struct PacketK {
+    static void *fn() { return reinterpret_cast<void *>(&k_queue_packet<FL>); }
+};
+
+void *queue_kernel(uint32_t fl, uint32_t refill_min) {
+    return refill_min >= 32u ? pick_fl<PacketK>(fl) : pick_fl<QueueK>(fl);
+}
 
 }  // namespace
 
@@ -419,7 +521,8 @@ cudaError_t QueueScratch::reserve(size_t n) {
     const size_t tiles = (m + kTileItems - 1) / kTileItems;
     cudaError_t e = cudaMalloc(&kv, m * sizeof(uint2));
     if (e == cudaSuccess) e = cudaMalloc(&kv2, m * sizeof(uint2));
-    if (e == cudaSuccess) e = cudaMalloc(&hist, (tiles + 1) * 256 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&hist, (tiles + kPasses) * 256 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(hist, 0, kPasses * 256 * sizeof(uint32_t));
     if (e == cudaSuccess) cap = n;
     return e;
 }
@@ -442,14 +545,17 @@ cudaError_t launch_queue(const TraceArgs &ta, const VxRay *rays, size_t n, VxHit
     if (t.sort) {
         const uint32_t tiles = (nn + kTileItems - 1) / kTileItems;
         const unsigned tb = (tiles + 3) / 4;
-        k_radix_keys<<<(nn + 255) / 256, 256, 0, s>>>(rays, nn, ta.ro[0], ta.ro[2], sc.kv);
+        // digit totals (256 per pass, zero between sorts), then the counts
+        uint32_t *totals = sc.hist, *counts = sc.hist + kPasses * 256u;
+        k_radix_keys<<<tiles, 256, 0, s>>>(rays, nn, ta.ro[0], ta.ro[2], sc.kv, tiles, counts,
+                                           totals);
         uint2 *in = sc.kv, *out = sc.kv2;
-        for (uint32_t shift = 0; shift < 32u; shift += 8u) {
-            k_radix_hist<<<tb, 128, 0, s>>>(in, nn, shift, tiles, sc.hist);
-            k_radix_rowsum<<<32, 256, 0, s>>>(sc.hist, tiles, sc.hist + (size_t)tiles * 256u);
-            k_radix_rowscan<<<256, 256, 0, s>>>(sc.hist, tiles, sc.hist + (size_t)tiles * 256u);
-            k_radix_scatter<<<tiles, 32 * kScatterWarps, 0, s>>>(in, nn, shift, tiles, sc.hist,
-                                                                 out);
+        for (uint32_t pass = 0; pass < kPasses; ++pass, totals += 256) {
+            const uint32_t shift = 8u * pass;
+            if (pass > 0) k_radix_hist<<<tb, 128, 0, s>>>(in, nn, shift, tiles, counts, totals);
+            k_radix_rowscan<<<256, 256, 0, s>>>(counts, tiles, totals);
+            k_radix_scatter<<<tiles, 32 * kScatterWarps, 0, s>>>(in, nn, shift, tiles, counts,
+                                                                 totals, out);
             std::swap(in, out);
         }
         order = in;
@@ -463,7 +569,7 @@ cudaError_t launch_queue(const TraceArgs &ta, const VxRay *rays, size_t n, VxHit
     q.shadow = shadow;
     q.work = sc.work;
     q.refill_min = (uint32_t)std::min(32, std::max(1, t.refill_min));
-    void *fn = queue_kernel((ta.p.flags & 7u) | pow2_bit(ta.w.d));
+    void *fn = queue_kernel((ta.p.flags & 7u) | pow2_bit(ta.w.d), q.refill_min);
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
