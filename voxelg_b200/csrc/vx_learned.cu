@@ -385,10 +385,9 @@ struct LearnedArgs {
 };
 
 template <uint32_t FL>
-// At least 6 CTAs per SM (up to 85 registers; 71 used): the learned frame
-// measured 0.203 ms against 0.211 ms at 7 and 0.212 ms at 8 (the register
-// budget of 8 forces the walk's state into fewer registers), 0.228 ms at 5.
-__global__ void __launch_bounds__(128, 6) k_learned(LearnedArgs la) {
+// At least 7 CTAs per SM: the learned frame measured 0.188 ms against 0.190 ms
+// at 6 and 0.197 ms at 5.
+__global__ void __launch_bounds__(128, 7) k_learned(LearnedArgs la) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t px = blockIdx.x * 16u + (warp & 1u) * 8u + (lane & 7u);
     const uint32_t py = blockIdx.y * 8u + (warp >> 1) * 4u + (lane >> 3);
@@ -450,16 +449,14 @@ __global__ void __launch_bounds__(128, 6) k_learned(LearnedArgs la) {
             uint32_t executed = 0;
             if (outcome != OUT_MISS) {
                 const uint32_t base = k.iters;
-                int r = WALK_CONT;
-                while (r == WALK_CONT) r = walk_step<FL, false, KIND_TRACE>(w, g, p, ro, k, h, bytes);
+                const int r = walk_to_end<FL, false, KIND_TRACE>(w, g, p, ro, k, h, bytes);
                 executed = k.iters - base;
-                if (r == WALK_END && k.iters >= k.cap && outcome != OUT_NONE) {
+                if (r != WALK_HIT && k.iters >= k.cap && outcome != OUT_NONE) {
                     // the inflated counter reached the cap: the plain DDA decides
                     fallback = 1;
                     set_miss(h);
                     walk_init(w.d, ro, KIND_TRACE, p, ox, oy, oz, dx, dy, dz, p.max_dist, k);
-                    while (walk_step<FL, false, KIND_TRACE>(w, g, p, ro, k, h, bytes) == WALK_CONT) {
-                    }
+                    walk_to_end<FL, false, KIND_TRACE>(w, g, p, ro, k, h, bytes);
                     executed += k.iters;
                 }
             }
