@@ -313,21 +313,8 @@ __device__ void worker(const ResArgs &a, uint4 *stage) {
             const float4 r0 = u4_as_f4(stage[2u * lane]), r1 = u4_as_f4(stage[2u * lane + 1u]);
             // kind in the low two bits, as vx_trace reads it
             const uint32_t kind = __float_as_uint(r1.w) & 3u;
-            uint64_t bytes = 0;
-            if (kind == 1u) {
-                uint32_t steps;
-                const bool occ = trace_any_ray<FL, false>(a.ta.w, a.ta.p, ro, r0.x, r0.y, r0.z,
-                                                          r0.w, r1.x, r1.y, r1.z, steps, bytes);
-                set_miss(h);
-                h.flags = occ ? 1u : 0u;
-                h.steps = steps;
-            } else if (kind == 2u) {
-                trace_no_water_ray<FL, false>(a.ta.w, a.ta.p, ro, r0.x, r0.y, r0.z, r0.w, r1.x,
-                                              r1.y, r1.z, h, bytes);
-            } else {
-                trace_ray<FL, false>(a.ta.w, a.ta.p, ro, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y,
-                                     r1.z, h, bytes);
-            }
+            trace_ray_of_kind<FL>(a.ta.w, a.ta.p, ro, kind, r0.x, r0.y, r0.z, r0.w, r1.x, r1.y,
+                                  r1.z, h);
         }
         __syncwarp();  // every lane has its ray out of the stage
         if (lane < cnt)
