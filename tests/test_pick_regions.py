@@ -99,3 +99,16 @@ def test_masks_that_do_not_hold(vg):
         dw.upload(a)
         assert check(vg, dw, ow, cams, dirs, (0, 0, 0), singles=50) > 100
     dw.close()
+
+
+@pytest.mark.parametrize("n", [0, 1, 31, 8193, 10001, 25001, 32769, 80001, 100001, 140000])
+def test_batch_sizes(vg, n):
+    """Either side of the sizes where a batch is cut into chunks and where the
+    lanes to a ray change."""
+    rng = np.random.default_rng(n)
+    ow = random_world(np.random.default_rng(2))
+    dw = vg.DeviceWorld(*ow.dims)
+    dw.upload(ow.a)
+    cams, dirs = rays(rng, n, ow.dims, (-37, 0, 70))
+    check(vg, dw, ow, cams, dirs, (-37, 0, 70), singles=min(n, 5))
+    dw.close()

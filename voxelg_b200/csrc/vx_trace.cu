@@ -414,20 +414,6 @@ __device__ __forceinline__ bool o1_in_window(const Dims &d, const int32_t v[3],
            (uint32_t)(v[2] - o[2]) < (uint32_t)d.vz;
 }
 
-__device__ __forceinline__ bool o1_in_solid(const DevWorld &w, const int32_t v[3],
-                                            const int32_t o[3]) {
-    const Dims &d = w.d;
-    if (!o1_in_window(d, v, o)) return false;
-    const int32_t sx = pos_mod(v[0], d.vx), sy = v[1], sz = pos_mod(v[2], d.vz);
-    const int64_t bi = (int64_t)(sx >> 2) + (int64_t)(sy >> 2) * d.bx +
-                       (int64_t)(sz >> 2) * d.bx * d.by;
-    const uint64_t occ = ld_occ(w, (uint64_t)bi);
-    if (occ == 0ull) return false;
-    const int vi = child_bit(sx & 3, sy & 3, sz & 3);
-    if (!bit64(occ, vi)) return false;
-    return ld_mat(w, (uint64_t)bi, (uint32_t)vi) != 33u;
-}
-
 // The walk of raycast(): direction normalised as glam 0.29.3's
 // normalize_or_zero (self * (1 / sqrt(dot))), window clip, start voxel
 // (raycast.rs:21-90).  False when the ray has no walk (zero direction,
@@ -475,71 +461,11 @@ __device__ __forceinline__ bool o1_start(const Dims &d, const int32_t o[3], cons
     return true;
 }
 
-// argmin_step, raycast.rs:92-103 (ties go to the lowest axis); -1: no axis
-__device__ __forceinline__ int o1_argmin_step(O1State &s) {
-    int a = -1;
-    float m = __int_as_float(0x7f800000);
-    if (s.step[0] != 0 && s.tm[0] < m) { a = 0; m = s.tm[0]; }
-    if (s.step[1] != 0 && s.tm[1] < m) { a = 1; m = s.tm[1]; }
-    if (s.step[2] != 0 && s.tm[2] < m) { a = 2; m = s.tm[2]; }
-    if (a == 0) { s.voxel[0] += s.step[0]; s.tm[0] += s.tdel[0]; }
-    else if (a == 1) { s.voxel[1] += s.step[1]; s.tm[1] += s.tdel[1]; }
-    else if (a == 2) { s.voxel[2] += s.step[2]; s.tm[2] += s.tdel[2]; }
-    return a;
-}
-
 __device__ __forceinline__ void o1_normal(const O1State &s, int last_axis, VxPickHit &res) {
     const int sa = last_axis == 0 ? s.step[0] : (last_axis == 1 ? s.step[1] : s.step[2]);
     if (last_axis == 0) res.normal[0] = -sa;
     else if (last_axis == 1) res.normal[1] = -sa;
     else if (last_axis == 2) res.normal[2] = -sa;
-}
-
-__global__ void __launch_bounds__(128) k_raycast(PickArgs pa, const float *__restrict__ cams,
-                                                 const float *__restrict__ dirs, size_t n,
-                                                 VxPickHit *out, int32_t *hit) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const Dims &d = pa.w.d;
-    const int32_t *o = pa.origin;
-    VxPickHit res;
-    res.voxel[0] = res.voxel[1] = res.voxel[2] = 0;
-    res.normal[0] = res.normal[1] = res.normal[2] = 0;
-    int32_t found = 0;
-    const float cam[3] = {cams[3 * i], cams[3 * i + 1], cams[3 * i + 2]};
-    const float din[3] = {dirs[3 * i], dirs[3 * i + 1], dirs[3 * i + 2]};
-    O1State s;
-    do {
-        if (!o1_start(d, o, cam, din, s)) break;
-        int last_axis = -1;
-        int steps_left = 4096;
-        bool dead = false;
-        // phase 1: leave the solids the start voxel is in
-        while (steps_left > 0 && o1_in_solid(pa.w, s.voxel, o)) {
-            const int ax = o1_argmin_step(s);
-            if (ax < 0) { dead = true; break; }
-            last_axis = ax;
-            steps_left--;
-            if (!o1_in_window(d, s.voxel, o)) { dead = true; break; }
-        }
-        if (dead) break;
-        // phase 2: the first solid non-fringe voxel
-        while (steps_left > 0) {
-            if (!o1_in_window(d, s.voxel, o)) break;
-            if (o1_in_solid(pa.w, s.voxel, o)) {
-                res.voxel[0] = s.voxel[0]; res.voxel[1] = s.voxel[1]; res.voxel[2] = s.voxel[2];
-                o1_normal(s, last_axis, res);
-                found = 1;
-                break;
-            }
-            const int ax = o1_argmin_step(s);
-            if (ax < 0) break;
-            last_axis = ax;
-            steps_left--;
-        }
-    } while (0);
-    out[i] = res;
-    hit[i] = found;
 }
 
 // The three crossing times of raycast()'s walk, for loops that step it many
@@ -557,117 +483,124 @@ __device__ __forceinline__ bool o1_times(const O1State &s, O1Times &t) {
     return t.x < inf || t.y < inf || t.z < inf;
 }
 
-// One ray with a whole warp (the single-call pick, where one thread's chain
-// of dependent steps and loads is the latency).  The voxel sequence of the
-// walk depends on arithmetic only: every lane takes the next 32 argmin steps
-// in registers and notes the axis of each as a bit, so element j of the walk
-// is the start plus the steps before bit j (three popcounts); each lane tests
-// its element (window, solid) at once, and raycast.rs's two phases are a few
-// bit scans over the answers.  The loads of a round leave before the steps of
-// the next, which cover their latency.  Element k of the walk is examined
-// with 4096 - k steps left: at most 128 rounds.
-// Lane 0 used to take the steps alone, through an indexed state and shared
-// memory, and the loads waited for them: 24 us a call on the device, 10 us now.
-__global__ void __launch_bounds__(32) k_raycast_warp(PickArgs pa, const float *__restrict__ cams,
-                                                     const float *__restrict__ dirs, VxPickHit *out,
-                                                     int32_t *hit) {
+// raycast() with G lanes to a ray (32: the single call).  The voxel sequence
+// of the walk depends on arithmetic only: every lane takes its ray's next G
+// argmin steps in registers and notes the axis of each as a bit, so element j
+// of the walk is the start plus the steps before bit j (three popcounts);
+// each lane tests its element (window, solid) at once, and raycast.rs's two
+// phases are a few bit scans over the answers.  The loads of a round leave
+// before the steps of the next, which cover their latency.  Element k of the
+// walk is examined with 4096 - k steps left: 4096 / G rounds at most.
+template <uint32_t G>
+__global__ void __launch_bounds__(128) k_raycast(PickArgs pa, const float *__restrict__ cams,
+                                                 const float *__restrict__ dirs, size_t n,
+                                                 VxPickHit *out, int32_t *hit) {
     constexpr unsigned FULL = 0xFFFFFFFFu;
-    const uint32_t lane = threadIdx.x;
+    constexpr unsigned GM = G == 32u ? FULL : (1u << (G & 31u)) - 1u;   // a group's bits
+    const uint32_t lane = threadIdx.x & 31u, g = lane & (G - 1u), at = lane - g;
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
     const Dims &d = pa.w.d;
     const int32_t *o = pa.origin;
-    // a single call passes its ray in the launch parameters: no read of
-    // host-mapped memory before the walk can start
-    const float *rc = cams ? cams : pa.ray, *rd = cams ? dirs : pa.ray + 3;
-    const float cam[3] = {rc[0], rc[1], rc[2]};
-    const float din[3] = {rd[0], rd[1], rd[2]};
-    VxPickHit res;
-    res.voxel[0] = res.voxel[1] = res.voxel[2] = 0;
-    res.normal[0] = res.normal[1] = res.normal[2] = 0;
-    int32_t found = 0;
+    int32_t found = 0, hx = 0, hy = 0, hz = 0;
+    int axis = 0;
     O1State s;
-    O1Times t;
-    if (o1_start(d, o, cam, din, s) && o1_times(s, t)) {   // same on every lane
-        const uint32_t before = (1u << lane) - 1u;
-        // the round's elements: bit j of ax / ay = the step after element j
-        // is along x / y (else z)
-        uint32_t ax = 0, ay = 0;
-        auto steps = [&]() {
-            ax = ay = 0;
+    O1Times t{0.f, 0.f, 0.f};
+    bool alive = false;
+    if (i < n) {
+        // a single call passes its ray in the launch parameters: no read of
+        // host-mapped memory before the walk can start
+        const float *rc = cams ? cams + 3 * i : pa.ray, *rd = cams ? dirs + 3 * i : pa.ray + 3;
+        const float cam[3] = {rc[0], rc[1], rc[2]};
+        const float din[3] = {rd[0], rd[1], rd[2]};
+        alive = o1_start(d, o, cam, din, s) && o1_times(s, t);   // same on a ray's lanes
+    }
+    const uint32_t before = (1u << g) - 1u;
+    // the round's elements: bit j of ax / ay = the step after element j is
+    // along x / y (else z)
+    uint32_t ax = 0, ay = 0;
+    auto steps = [&]() {
+        ax = ay = 0;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const bool px = !(t.y < t.x) && !(t.z < t.x);
-                const bool py = !px && !(t.z < t.y);
-                if (px) { t.x += s.tdel[0]; ax |= 1u << j; }
-                else if (py) { t.y += s.tdel[1]; ay |= 1u << j; }
-                else t.z += s.tdel[2];
-            }
-        };
-        int32_t vx = s.voxel[0], vy = s.voxel[1], vz = s.voxel[2];   // element 0 of the round
-        uint32_t last = 0u;            // axis of the step into element 0 (rounds after the first)
-        bool walking = false;          // phase 2: past the solids the start is in
-        steps();
-        for (int32_t base = 0; base < 4096; base += 32) {
-            const uint32_t az = ~(ax | ay);
-            const int32_t v[3] = {vx + s.step[0] * (int32_t)__popc(ax & before),
-                                  vy + s.step[1] * (int32_t)__popc(ay & before),
-                                  vz + s.step[2] * (int32_t)__popc(az & before)};
-            // occupancy word and material byte of the element, both loads out
-            // before either is used
-            const bool inwin = o1_in_window(d, v, o);
-            uint64_t occ = 0ull;
-            uint32_t mat = 0u;
-            int vi = 0;
-            if (inwin) {
-                const int32_t sx = pos_mod(v[0], d.vx), sy = v[1], sz = pos_mod(v[2], d.vz);
-                const uint64_t bi = (uint64_t)((int64_t)(sx >> 2) + (int64_t)(sy >> 2) * d.bx +
-                                               (int64_t)(sz >> 2) * d.bx * d.by);
-                vi = child_bit(sx & 3, sy & 3, sz & 3);
-                occ = ld_occ(pa.w, bi);
-                mat = ld_mat(pa.w, bi, (uint32_t)vi);
-            }
-            const uint32_t rx = ax, ry = ay;
-            const int32_t nx = vx + s.step[0] * (int32_t)__popc(ax),
-                          ny = vy + s.step[1] * (int32_t)__popc(ay),
-                          nz = vz + s.step[2] * (int32_t)__popc(az);
-            steps();                   // the next round's, while the loads are out
-            const unsigned win = __ballot_sync(FULL, inwin);
-            const unsigned sol = __ballot_sync(FULL, bit64(occ, vi) && mat != 33u);
-            unsigned look = FULL;      // elements phase 2 examines
-            bool end = false;
-            if (!walking) {
-                // phase 1: the first element that is not solid
-                const int k = __ffs(~sol) - 1;
-                if (k >= 0) {
-                    walking = true;
-                    end = !((win >> k) & 1u);   // its steps left the window
-                    look = FULL << k;
-                } else {
-                    look = 0u;
-                }
-            }
-            // phase 2: the first element outside the window or solid
-            const unsigned stop = look & (~win | sol);
-            if (end || stop) {
-                const int k = __ffs(stop) - 1;
-                if (!end && ((win >> k) & 1u)) {
-                    found = 1;
-                    res.voxel[0] = __shfl_sync(FULL, v[0], k);
-                    res.voxel[1] = __shfl_sync(FULL, v[1], k);
-                    res.voxel[2] = __shfl_sync(FULL, v[2], k);
-                    uint32_t axis = last;
-                    if (k > 0) axis = (rx >> (k - 1)) & 1u ? 0u : ((ry >> (k - 1)) & 1u ? 1u : 2u);
-                    o1_normal(s, (int)axis, res);
-                }
-                break;
-            }
-            last = rx >> 31 ? 0u : (ry >> 31 ? 1u : 2u);
-            vx = nx; vy = ny; vz = nz;
+        for (uint32_t j = 0; j < G; ++j) {
+            const bool px = !(t.y < t.x) && !(t.z < t.x);
+            const bool py = !px && !(t.z < t.y);
+            if (px) { t.x += s.tdel[0]; ax |= 1u << j; }
+            else if (py) { t.y += s.tdel[1]; ay |= 1u << j; }
+            else t.z += s.tdel[2];
         }
+    };
+    int32_t vx = s.voxel[0], vy = s.voxel[1], vz = s.voxel[2];   // element 0 of the round
+    uint32_t last = 0u;            // axis of the step into element 0 (rounds after the first)
+    bool walking = false;          // phase 2: past the solids the start is in
+    steps();
+    for (int32_t base = 0; base < 4096 && __any_sync(FULL, alive); base += (int32_t)G) {
+        const uint32_t az = GM & ~(ax | ay);
+        const int32_t v[3] = {vx + s.step[0] * (int32_t)__popc(ax & before),
+                              vy + s.step[1] * (int32_t)__popc(ay & before),
+                              vz + s.step[2] * (int32_t)__popc(az & before)};
+        const bool inwin = alive && o1_in_window(d, v, o);
+        uint64_t occ = 0ull;
+        uint64_t bi = 0ull;
+        uint32_t mat = 0u;
+        int vi = 0;
+        if (inwin) {
+            const int32_t sx = pos_mod(v[0], d.vx), sy = v[1], sz = pos_mod(v[2], d.vz);
+            bi = (uint64_t)((int64_t)(sx >> 2) + (int64_t)(sy >> 2) * d.bx +
+                            (int64_t)(sz >> 2) * d.bx * d.by);
+            vi = child_bit(sx & 3, sy & 3, sz & 3);
+            occ = ld_occ(pa.w, bi);
+            // alone on the device, the material byte leaves with the word
+            if (G == 32u) mat = ld_mat(pa.w, bi, (uint32_t)vi);
+        }
+        const uint32_t rx = ax, ry = ay;
+        const int32_t nx = vx + s.step[0] * (int32_t)__popc(ax),
+                      ny = vy + s.step[1] * (int32_t)__popc(ay),
+                      nz = vz + s.step[2] * (int32_t)__popc(az);
+        steps();                   // the next round's, while the loads are out
+        bool solid = bit64(occ, vi);
+        if (G != 32u && solid) mat = ld_mat(pa.w, bi, (uint32_t)vi);
+        solid = solid && mat != 33u;
+        const unsigned win = (__ballot_sync(FULL, inwin) >> at) & GM;
+        const unsigned sol = (__ballot_sync(FULL, solid) >> at) & GM;
+        unsigned look = GM;        // elements phase 2 examines
+        bool end = false;
+        if (!walking) {
+            // phase 1: the first element that is not solid
+            const unsigned open = GM & ~sol;
+            if (open != 0u) {
+                const int k = __ffs((int)open) - 1;
+                walking = true;
+                end = !((win >> k) & 1u);   // its steps left the window
+                look = GM & (FULL << k);
+            } else {
+                look = 0u;
+            }
+        }
+        // phase 2: the first element outside the window or solid
+        const unsigned stop = look & (~win | sol);
+        const bool over = alive && (end || stop != 0u);
+        const int k = stop != 0u ? __ffs((int)stop) - 1 : 0;
+        const int32_t ex = __shfl_sync(FULL, v[0], (int)at + k), ey = __shfl_sync(FULL, v[1], (int)at + k),
+                      ez = __shfl_sync(FULL, v[2], (int)at + k);
+        if (over) {
+            alive = false;
+            if (!end && ((win >> k) & 1u)) {
+                found = 1;
+                hx = ex; hy = ey; hz = ez;
+                axis = (int)last;
+                if (k > 0) axis = (rx >> (k - 1)) & 1u ? 0 : ((ry >> (k - 1)) & 1u ? 1 : 2);
+            }
+        }
+        last = (rx >> (G - 1u)) & 1u ? 0u : ((ry >> (G - 1u)) & 1u ? 1u : 2u);
+        vx = nx; vy = ny; vz = nz;
     }
-    if (lane == 0) {
-        *out = res;
-        *hit = found;
-    }
+    if (g != 0u || i >= n) return;
+    VxPickHit res;
+    res.voxel[0] = hx; res.voxel[1] = hy; res.voxel[2] = hz;
+    res.normal[0] = res.normal[1] = res.normal[2] = 0;
+    if (found) o1_normal(s, axis, res);
+    out[i] = res;
+    hit[i] = found;
 }
 
 // raycast() over the pyramid: the same walk, one thread per ray, that tests
@@ -679,7 +612,7 @@ __global__ void __launch_bounds__(32) k_raycast_warp(PickArgs pa, const float *_
 // add and a subtraction.  Needs masks that hold for the bricks (VxWorld's
 // masks_hold); k_raycast reads the occupancy of every voxel instead, which is
 // what raycast.rs does.
-// 200,000 picks over the demo world (114 steps and 17 regions a ray): 520 us
+// 200,000 picks over the demo world (114 steps and 17 regions a ray): 482 us
 // voxel by voxel, 246 us here.  Rays of unlike length and place share a warp,
 // so it is bound by the lanes that wait; taking the steps of a region a few
 // at a time (3 to 16) between looks, or with votes to keep the warp together,
@@ -1121,7 +1054,7 @@ cudaError_t launch_raycast_one(const DevWorld &w, const int32_t origin[3], const
         pa.ray[k] = cam[k];
         pa.ray[3 + k] = dir[k];
     }
-    k_raycast_warp<<<1, 32, 0, s>>>(pa, nullptr, nullptr, out, hit);
+    k_raycast<32><<<1, 32, 0, s>>>(pa, nullptr, nullptr, 1, out, hit);
     return cudaGetLastError();
 }
 
@@ -1132,13 +1065,21 @@ cudaError_t launch_raycast(const DevWorld &w, const int32_t origin[3], const flo
     PickArgs pa;
     pa.w = w;
     pa.origin[0] = origin[0]; pa.origin[1] = origin[1]; pa.origin[2] = origin[2];
-    if (n == 1) {
-        k_raycast_warp<<<1, 32, 0, s>>>(pa, cams, dirs, out, hit);
-        return cudaGetLastError();
-    }
-    const unsigned blocks = (unsigned)((n + 127) / 128);
-    if (masks_hold) k_raycast_skip<<<blocks, 128, 0, s>>>(pa, cams, dirs, n, out, hit);
-    else k_raycast<<<blocks, 128, 0, s>>>(pa, cams, dirs, n, out, hit);
+    // Lanes to a ray: all 32 for the shortest time of a few, fewer as the
+    // rays fill the device, and one ray a thread over the pyramid for many.
+    // us at G = 32 / 16 / 8 / 4 and by regions (demo world, 114 steps a ray):
+    //   1,000    21 / 27 / 39 / 60, 133      50,000  148 / 131 / 110 / 118, 158
+    //   8,000    38 / 39 / 48 / 70, 154     100,000  279 / 240 / 191 / 181, 182
+    //   200,000  546 / 463 / 350 / 312, 246; 1,000,000  - / - / 1623 / 1367, 789
+    // (one ray a thread voxel by voxel: 277, 326, 369, 383, 482, 1521)
+    auto lanes = [&](auto kernel, unsigned g) {
+        kernel<<<(unsigned)((n * g + 127) / 128), 128, 0, s>>>(pa, cams, dirs, n, out, hit);
+    };
+    if (n <= 10000) lanes(k_raycast<32>, 32);
+    else if (n <= 25000) lanes(k_raycast<16>, 16);
+    else if (n <= 80000) lanes(k_raycast<8>, 8);
+    else if (!masks_hold || n <= 100000) lanes(k_raycast<4>, 4);
+    else k_raycast_skip<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(pa, cams, dirs, n, out, hit);
     return cudaGetLastError();
 }
 
