@@ -301,6 +301,13 @@ int vx_raycast(VxWorld *w, const float cam[3], const float dir[3], const int32_t
 int vx_raycast_batch(VxWorld *w, const int32_t origin[3], const float *cams_dev,
                      const float *dirs_dev, size_t n, VxPickHit *out_dev, int32_t *hit_dev,
                      void *stream);
+/* The same over host arrays: the results are in out_host / hit_host when the
+ * call returns.  Rays go to the device in chunks, each traced and its results
+ * copied back while the next is on its way; results land fastest in
+ * page-locked memory.  The device buffers are the world's. */
+int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams_host,
+                          const float *dirs_host, size_t n, VxPickHit *out_host,
+                          int32_t *hit_host);
 /* Batched generic rays (trace / trace_any / trace_no_water) over device
  * arrays; origin is the loaded-window corner. */
 int vx_trace(VxWorld *w, const int32_t origin[3], const VxRay *rays_dev, size_t n,
@@ -331,7 +338,7 @@ int vx_render_primary_rows(VxWorld *w, const VxCamera *cam, const VxTraceParams 
                            void *stream);
 /* Same frame through host buffers: the records are copied to rec_host /
  * shadow_host (pinned memory recommended) before the call returns.  The
- * frame renders in four row bands, each copied while the next renders. */
+ * frame renders in six row bands, each copied while the next ones render. */
 int vx_render_primary_host(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
                            VxHitRecord *rec_host, VxShadowRecord *shadow_host);
 /* The same, for frame pipelines: enqueues the frame and returns.  Its

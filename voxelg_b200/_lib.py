@@ -174,6 +174,7 @@ SIGNATURES = [
     ("vx_world_get_tuning", C.c_int, [_vp, _P(VxTuning)]),
     ("vx_raycast", C.c_int, [_vp, _P(C.c_float), _P(C.c_float), _P(C.c_int32), _P(VxPickHit)]),
     ("vx_raycast_batch", C.c_int, [_vp, _P(C.c_int32), _vp, _vp, C.c_size_t, _vp, _vp, _vp]),
+    ("vx_raycast_batch_host", C.c_int, [_vp, _P(C.c_int32), _vp, _vp, C.c_size_t, _vp, _vp]),
     ("vx_trace", C.c_int, [_vp, _P(C.c_int32), _vp, C.c_size_t, _P(VxTraceParams), _vp, _vp]),
     ("vx_render_primary", C.c_int, [_vp, _P(VxCamera), _P(VxTraceParams), _vp, _vp, _vp]),
     ("vx_render_primary_host", C.c_int, [_vp, _P(VxCamera), _P(VxTraceParams), _vp, _vp]),

@@ -61,8 +61,15 @@ struct VxWorld {
     cudaStream_t copy_stream = nullptr;
     uint32_t *d_gate_idx = nullptr;  // staging of vx_project_dirty
     size_t gate_cap = 0;
+    uint8_t *pick_buf = nullptr;     // vx_raycast_batch_host: results, cameras, directions
+    size_t pick_cap = 0;
+    cudaStream_t pick_in = nullptr;  // its copies in, every other chunk's traces, events
+    cudaStream_t pick_b = nullptr;
+    cudaEvent_t pick_ev[4] = {}, pick_fork = nullptr;
     vx::QueueScratch qs;             // scratch of vx_queue_run / vx_queue_autotune
-    cudaEvent_t band_ev[4] = {};    // one per row band (kSyncBands at most)
+    cudaEvent_t band_ev[6] = {};    // one per row band (kSyncBands at most)
+    cudaStream_t band_stream = nullptr;  // every other band of a synchronous host frame
+    cudaEvent_t band_fork = nullptr;
     VxTuning tuning{0, {0, 0, 0, 0, 0, 0, 0}};
     // chunk generator state: the world chunk each storage-chunk slot holds
     // (3 ints per slot, empty until a window is filled), its seed and origin
@@ -187,7 +194,7 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 // renders while the previous one copies), so one band, i.e. the fewest
 // copies, is fastest there: 1.18 ms per 1080p frame against 1.23 ms with 8
 // bands, where the copy engine spends a few microseconds per copy.
-constexpr uint32_t kSyncBands = 4;
+constexpr uint32_t kSyncBands = 6;
 constexpr uint32_t kAsyncBands = 1;
 
 int use_device(VxWorld *w) {
@@ -225,6 +232,12 @@ void free_world(VxWorld *w) {
     if (w->pick) cudaFreeHost(w->pick);
     cudaFree(w->d_work);
     cudaFree(w->d_gate_idx);
+    cudaFree(w->pick_buf);
+    for (auto &e : w->pick_ev)
+        if (e) cudaEventDestroy(e);
+    if (w->pick_fork) cudaEventDestroy(w->pick_fork);
+    if (w->pick_in) cudaStreamDestroy(w->pick_in);
+    if (w->pick_b) cudaStreamDestroy(w->pick_b);
     cudaFree(w->d_gen);
     cudaFree(w->d_edits);
     cudaFree(w->bdf);
@@ -242,6 +255,7 @@ void free_world(VxWorld *w) {
         if (b.done) cudaEventDestroy(b.done);
     }
     if (w->dirty_last) cudaEventDestroy(w->dirty_last);
+    if (w->band_stream) cudaStreamSynchronize(w->band_stream);
     if (w->copy_stream) cudaStreamSynchronize(w->copy_stream);
     for (int i = 0; i < 2; ++i) {
         cudaFree(w->hrec[i]);
@@ -254,6 +268,8 @@ void free_world(VxWorld *w) {
         if (e) cudaEventDestroy(e);
     for (auto &e : w->band_ev)
         if (e) cudaEventDestroy(e);
+    if (w->band_fork) cudaEventDestroy(w->band_fork);
+    if (w->band_stream) cudaStreamDestroy(w->band_stream);
     if (w->copy_stream) cudaStreamDestroy(w->copy_stream);
     if (w->stream) cudaStreamDestroy(w->stream);
 }
@@ -1264,6 +1280,71 @@ int vx_raycast_batch(VxWorld *w, const int32_t origin[3], const float *cams_dev,
     return VX_OK;
 }
 
+int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams_host,
+                          const float *dirs_host, size_t n, VxPickHit *out_host,
+                          int32_t *hit_host) {
+    vx::Range nvtx_range("vx_raycast_batch_host");
+    if (!w || !origin || (n > 0 && (!cams_host || !dirs_host || !out_host || !hit_host))) {
+        vx::set_error("vx_raycast_batch_host: null argument");
+        return VX_ERR_INVALID;
+    }
+    if (!vx::origin_ok(origin, "vx_raycast_batch_host")) return VX_ERR_INVALID;
+    if (n == 0) return VX_OK;
+    int rc = use_device(w);
+    if (rc != VX_OK) return rc;
+    std::lock_guard<std::mutex> lk(w->mu);
+    rc = ensure(&w->pick_buf, &w->pick_cap, n * (sizeof(VxPickHit) + 24 + sizeof(int32_t)));
+    if (rc != VX_OK) return rc;
+    VxPickHit *out = reinterpret_cast<VxPickHit *>(w->pick_buf);
+    float *cams = reinterpret_cast<float *>(out + n), *dirs = cams + 3 * n;
+    int32_t *hit = reinterpret_cast<int32_t *>(dirs + 3 * n);
+    if (!w->pick_in) {
+        VX_CK(cudaStreamCreateWithFlags(&w->pick_in, cudaStreamNonBlocking));
+        VX_CK(cudaStreamCreateWithFlags(&w->pick_b, cudaStreamNonBlocking));
+        for (auto &ev : w->pick_ev) VX_CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        VX_CK(cudaEventCreateWithFlags(&w->pick_fork, cudaEventDisableTiming));
+    }
+    // after what the world's stream holds (updates of the world)
+    VX_CK(cudaEventRecord(w->pick_fork, w->stream));
+    VX_CK(cudaStreamWaitEvent(w->pick_b, w->pick_fork, 0));
+    // Copies in on a stream of their own; a chunk is traced and returned while
+    // the next one comes in, on two streams in turn, since a chunk's launch
+    // ends with its few longest rays.  200,000 rays from and to pageable
+    // memory took 1.07 ms as whole copies one after the other, 0.57 ms so.
+    // A chunk is not worth its launches below some thousand rays.
+    constexpr size_t kChunks = sizeof(w->pick_ev) / sizeof(w->pick_ev[0]);
+    const size_t chunk = std::max<size_t>((n + kChunks - 1) / kChunks, 8192);
+    cudaError_t e = cudaSuccess;
+    auto ok = [&e](cudaError_t r) {
+        if (e == cudaSuccess) e = r;
+        return e == cudaSuccess;
+    };
+    size_t k = 0;
+    for (size_t a = 0; a < n && e == cudaSuccess; a += chunk, ++k) {
+        const size_t m = std::min(chunk, n - a);
+        const cudaStream_t s = (k & 1u) ? w->pick_b : w->stream;
+        ok(cudaMemcpyAsync(cams + 3 * a, cams_host + 3 * a, m * 12, cudaMemcpyHostToDevice,
+                           w->pick_in)) &&
+            ok(cudaMemcpyAsync(dirs + 3 * a, dirs_host + 3 * a, m * 12, cudaMemcpyHostToDevice,
+                               w->pick_in)) &&
+            ok(cudaEventRecord(w->pick_ev[k], w->pick_in)) &&
+            ok(cudaStreamWaitEvent(s, w->pick_ev[k], 0)) &&
+            ok(vx::launch_raycast(w->dw, origin, cams + 3 * a, dirs + 3 * a, m, out + a,
+                                  hit + a, w->masks_hold, s)) &&
+            ok(cudaMemcpyAsync(out_host + a, out + a, m * sizeof(VxPickHit),
+                               cudaMemcpyDeviceToHost, s)) &&
+            ok(cudaMemcpyAsync(hit_host + a, hit + a, m * sizeof(int32_t),
+                               cudaMemcpyDeviceToHost, s));
+    }
+    // nothing may be on its way to or from the caller's arrays after this
+    for (cudaStream_t s : {w->pick_in, w->pick_b, w->stream}) {
+        const cudaError_t r = cudaStreamSynchronize(s);
+        ok(r);
+    }
+    VX_CK(e);
+    return VX_OK;
+}
+
 int vx_trace(VxWorld *w, const int32_t origin[3], const VxRay *rays_dev, size_t n,
              const VxTraceParams *p, VxHitRecord *out_dev, void *stream) {
     vx::Range nvtx_range("vx_trace");
@@ -1573,6 +1654,8 @@ int enqueue_host_frame(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
     if (!w->copy_stream) {
         VX_CK(cudaStreamCreateWithFlags(&w->copy_stream, cudaStreamNonBlocking));
         for (auto &e : w->band_ev) VX_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        VX_CK(cudaStreamCreateWithFlags(&w->band_stream, cudaStreamNonBlocking));
+        VX_CK(cudaEventCreateWithFlags(&w->band_fork, cudaEventDisableTiming));
     }
     if (!w->copy_done[0]) {
         for (auto &e : w->copy_done) VX_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1599,24 +1682,31 @@ int enqueue_host_frame(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
         fa.beam = w->beam;
         VX_CK(vx::launch_beam(fa, w->beam, w->stream));
     }
+    // Bands go to two streams in turn: a band ends with its few longest rays,
+    // and the next one fills the device meanwhile.
+    if (nb > 1) {
+        VX_CK(cudaEventRecord(w->band_fork, w->stream));
+        VX_CK(cudaStreamWaitEvent(w->band_stream, w->band_fork, 0));
+    }
     for (uint32_t b = 0; b < nb; ++b) {
+        const cudaStream_t bs = (b & 1u) ? w->band_stream : w->stream;
         fa.y0 = std::min(fa.H, b * band);
         fa.y1 = std::min(fa.H, (b + 1) * band);
         if (fa.work) fa.y0 = 0, fa.y1 = fa.H;
         if (fa.y1 <= fa.y0) break;
-        VX_CK(vx::launch_primary(fa, w->stream));
+        VX_CK(vx::launch_primary(fa, bs));
         const size_t r0 = (size_t)fa.y0 * fa.W, rn = (size_t)(fa.y1 - fa.y0) * fa.W;
         if (packed) {
             const uint32_t wx = (uint32_t)w->dw.d.vx, wy = (uint32_t)w->dw.d.vy;
             if (compact)
                 VX_CK(vx::launch_pack_compact(fa.rec, fa.shadow, r0, rn, fa.ta.ro, wx, wy,
                                               reinterpret_cast<VxCompactRecord *>(w->hpk[buf]),
-                                              fa.ta.w.fault, w->stream));
+                                              fa.ta.w.fault, bs));
             else
                 VX_CK(vx::launch_pack(fa.rec, fa.shadow, r0, rn, fa.ta.ro, wx, wy, w->hpk[buf],
-                                      w->stream));
+                                      bs));
         }
-        VX_CK(cudaEventRecord(w->band_ev[b], w->stream));
+        VX_CK(cudaEventRecord(w->band_ev[b], bs));
         VX_CK(cudaStreamWaitEvent(w->copy_stream, w->band_ev[b], 0));
         if (compact) {
             VX_CK(cudaMemcpyAsync(compact_host + r0,
@@ -1636,6 +1726,8 @@ int enqueue_host_frame(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
             VX_CK(cudaMemcpyAsync(shadow_host + r0, fa.shadow + r0, rn * sizeof(VxShadowRecord),
                                   cudaMemcpyDeviceToHost, w->copy_stream));
     }
+    // what follows on the world's stream follows every band
+    for (uint32_t b = 1; b < nb; b += 2) VX_CK(cudaStreamWaitEvent(w->stream, w->band_ev[b], 0));
     VX_CK(cudaEventRecord(w->copy_done[buf], w->copy_stream));
     ++w->host_frames;
     return VX_OK;
