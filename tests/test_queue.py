@@ -161,3 +161,26 @@ def test_queue_sorted_sizes(gpu, c1_oracle_world, n):
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy(), want.view(np.uint8))
     assert np.array_equal(sh.cpu().numpy(), wsh.view(np.uint8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 1023, 1024, 1025, 4097, 300_000])
+def test_sorted_queue_at_bucket_edges(gpu, n):
+    """Few and many rays (the sort's bucket count follows their number), all
+    in one bucket or spread over all of them: every record equals vx_trace."""
+    import torch
+    import voxelg_b200.queue as q
+    vg, dw = gpu
+    rng = np.random.default_rng(n)
+    p = vg.default_params(7)
+    for spread in (False, True):
+        rays = np.zeros(n, po.RAY)
+        rays["org"] = rng.uniform([0, 60, 0], [512, 200, 512], (n, 3)) if spread else (256, 150, 256)
+        d = rng.normal(size=(n, 3)) if spread else np.tile([0.3, -0.5, 0.8], (n, 1))
+        rays["dir"] = d / np.linalg.norm(d, axis=1, keepdims=True)
+        rays["tmax"] = 300.0
+        rays["kind"] = rng.integers(0, 4, n) if spread else 0
+        _, out, _ = q.run(dw, rays, p, with_shadow=False)
+        want = vg.trace(dw, rays, p)
+        torch.cuda.synchronize()
+        assert torch.equal(out, want), (n, spread)

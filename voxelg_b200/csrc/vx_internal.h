@@ -201,9 +201,9 @@ cudaError_t launch_apply_dirty(const DevWorld &w, const uint32_t *idx, const VxB
 // work counters, coherence-sort keys / permutation / histogram, fingerprint.
 struct QueueScratch {
     uint32_t *work = nullptr;
-    uint2 *kv = nullptr;          // coherence sort: (key, ray) pairs
-    uint2 *kv2 = nullptr;         // and their ping-pong partner
-    uint32_t *hist = nullptr;     // per-tile digit counts
+    uint2 *place = nullptr;       // coherence sort: each ray's bucket and place in it
+    uint32_t *order = nullptr;    // ray numbers by key
+    uint32_t *counts = nullptr;   // rays per bucket, then each bucket's first place
     unsigned long long *fp = nullptr;
     size_t cap = 0;
     cudaError_t reserve(size_t n);

@@ -7,13 +7,13 @@
 // that hits and carries VX_RAY_SPAWN_SHADOW continues in the same lane with
 // its shadow ray (raymarch.wgsl:3953-3994).  Lanes of a warp refill together
 // once `refill_min` of them are idle (a lone refill would stall 31 lanes
-// through a ray set-up).  Optionally the queue is first reordered by a 32-bit
+// through a ray set-up).  Optionally the queue is first reordered by a 22-bit
 // coherence key -- kind, then the direction on a 1024x1024 octahedral grid in
-// Morton order, then the 64-voxel origin cell -- with a stable LSD radix sort
-// (four 8-bit passes), so that a warp's rays head the same way from nearby
-// origins: rays of one camera fall into pixel-sized direction cells, the
-// rays of one probe site stay together.  Results do not depend on any of
-// these choices; the autotuner checks that and keeps the fastest.
+// Morton order, crossed with the 64-voxel origin cell -- by a counting sort,
+// so that a warp's rays head the same way from nearby origins: rays of one
+// camera fall into pixel-sized direction cells, the rays of one probe site
+// stay together.  Results do not depend on any of these choices; the
+// autotuner checks that and keeps the fastest.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,13 +28,10 @@
 namespace vx {
 namespace {
 
-constexpr uint32_t kTileItems = 2048;   // radix sort: items per warp-tile
-constexpr uint32_t kPasses = 4;         // 8-bit digits of the key
-
 struct QueueArgs {
     TraceArgs ta;
     const VxRay *rays;
-    const uint2 *order;       // sorted (key, ray) pairs or nullptr (identity order)
+    const uint32_t *order;    // ray numbers by key, or nullptr (identity order)
     uint32_t n;
     VxHitRecord *out;
     VxShadowRecord *shadow;   // shadow records of spawning rays, or nullptr
@@ -108,7 +105,7 @@ __global__ void __launch_bounds__(256) k_queue(QueueArgs q) {
                     item = DONE;
                 } else {
                     item = slot;
-                    ray = q.order ? __ldg(q.order + slot).y : slot;
+                    ray = q.order ? __ldg(q.order + slot) : slot;
                     float dx, dy, dz, tmax;
                     load_ray(q.rays, ray, ox, oy, oz, dx, dy, dz, tmax, rkind);
                     shadow_phase = false;
@@ -190,7 +187,7 @@ __global__ void __launch_bounds__(256, 3) k_queue_packet(QueueArgs q) {
         if (lane == 0) next = atomicAdd(q.work, 32u);
         const uint32_t slot = base + lane;
         if (slot < q.n) {
-            const uint32_t ray = q.order ? __ldg(q.order + slot).y : slot;
+            const uint32_t ray = q.order ? __ldg(q.order + slot) : slot;
             float ox, oy, oz, dx, dy, dz, tmax;
             uint32_t rkind;
             load_ray(q.rays, ray, ox, oy, oz, dx, dy, dz, tmax, rkind);
@@ -231,9 +228,24 @@ __global__ void __launch_bounds__(256, 3) k_queue_packet(QueueArgs q) {
     }
 }
 
-// ---- coherence reorder: stable LSD radix sort of a 32-bit key
-// key = kind(2) | Morton(octahedral direction, 10+10 bits) | origin cell(10:
-// 64-voxel cells, 4 bits each in x and z, 2 in y)
+// ---- coherence reorder: a counting sort by a key of at most 22 bits
+// key = kind(2) | Morton(octahedral direction, 10+10 bits) with the origin's
+// 64-voxel cell XORed into its low 10 bits: rays of one origin stay in Morton
+// order up to a reflection of blocks of 1024 cells, rays of one direction are
+// parted by cell.  A launch of few rays drops low bits, to about four buckets
+// a ray.
+//
+// What bounds it: the rays are read once (32 bytes each; the 1080p mix's 98 MB
+// take 15 us at the copy rate); all else is in L2.  One pass counts, and the
+// count a ray finds is its place in its bucket; the counts are summed up; one
+// pass writes each ray's number to its place, 4 scattered bytes.  The order
+// within a bucket is as the atomics fall: the records do not depend on it.
+// 1080p mix, launches one by one: 212 us as four passes of a stable radix sort
+// over 32-bit keys (histogram, row scan, scatter by digit runs each), 97 us
+// so; the walks lose 15 us to the coarser order, the queue gains 87 (738 us to
+// 651; 21 and 20 key bits: 666 and 660).
+constexpr uint32_t kKeyBits = 22;
+constexpr uint32_t kScanItems = 4096;    // buckets a CTA sums and scans
 
 __device__ __forceinline__ uint32_t spread_bits(uint32_t x) {   // 10 bits -> even bits
     x &= 0x3FFu;
@@ -267,61 +279,27 @@ __device__ __forceinline__ uint32_t ray_key(const VxRay *rays, uint32_t i, int32
         return ((uint32_t)c >> 6) & 15u;
     };
     const uint32_t oc = cell(ox, rox) | (cell(oz, roz) << 4) | ((cell(oy, 0) & 3u) << 8);
-    return ((kind & 3u) << 30) | (morton << 10) | oc;
+    return ((kind & 3u) << 20) | (morton ^ oc);
 }
 
-// (key, ray) pairs of a 2048-ray tile per CTA, and the tile's counts of the
-// first digit on the way (k_radix_hist counts the others').  All counts also
-// go to the digit's total over the tiles, from which k_radix_rowscan forms its
-// base: a launch per pass that summed the rows, and a first k_radix_hist, went
-// (24 us of the 1080p mix).
-// Shorter keys were no gain: 24 bits save a pass (about 45 us) and cost 75-90
-// in the walks, whose rays sort less well; 22 or 24 direction bits change
-// nothing.
-__global__ void __launch_bounds__(256) k_radix_keys(const VxRay *rays, uint32_t n, int32_t rox,
-                                                    int32_t roz, uint2 *kv, uint32_t tiles,
-                                                    uint32_t *counts, uint32_t *totals) {
-    __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0u;
-    __syncthreads();
-    const uint32_t begin = blockIdx.x * kTileItems, end = min(n, begin + kTileItems);
-    for (uint32_t i = begin + threadIdx.x; i < end; i += 256u) {
-        const uint32_t key = ray_key(rays, i, rox, roz);
-        kv[i] = make_uint2(key, i);
-        atomicAdd(&h[key & 255u], 1u);
-    }
-    __syncthreads();
-    const uint32_t t = h[threadIdx.x];
-    counts[threadIdx.x * tiles + blockIdx.x] = t;
-    if (t != 0u) atomicAdd(totals + threadIdx.x, t);
+// Each ray's bucket and its place in it.  Lanes of a warp with one bucket
+// share an atomic, so rays that all share a few keys do not queue up.
+__global__ void __launch_bounds__(256) k_sort_count(const VxRay *rays, uint32_t n, int32_t rox,
+                                                    int32_t roz, uint32_t shift, uint32_t *counts,
+                                                    uint2 *place) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = i < n;
+    const unsigned lanes = __ballot_sync(0xFFFFFFFFu, live);
+    if (!live) return;
+    const uint32_t b = ray_key(rays, i, rox, roz) >> shift, lane = threadIdx.x & 31u;
+    const unsigned peers = __match_any_sync(lanes, b);
+    const int leader = __ffs((int)peers) - 1;
+    uint32_t first = 0;
+    if ((int)lane == leader) first = atomicAdd(counts + b, (uint32_t)__popc(peers));
+    first = __shfl_sync(lanes, first, leader);
+    place[i] = make_uint2(b, first + (uint32_t)__popc(peers & ((1u << lane) - 1u)));
 }
 
-// Per warp-tile histogram of one 8-bit digit: counts[digit * tiles + tile].
-__global__ void __launch_bounds__(128) k_radix_hist(const uint2 *kv, uint32_t n,
-                                                    uint32_t shift, uint32_t tiles,
-                                                    uint32_t *counts, uint32_t *totals) {
-    __shared__ uint32_t h[4][256];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    for (uint32_t d = lane; d < 256u; d += 32u) h[warp][d] = 0u;
-    __syncwarp();
-    const uint32_t tile = blockIdx.x * 4u + warp;
-    if (tile < tiles) {
-        const uint32_t end = min(n, (tile + 1u) * kTileItems);
-        for (uint32_t i = tile * kTileItems + lane; i < end; i += 32u)
-            atomicAdd(&h[warp][(kv[i].x >> shift) & 255u], 1u);
-        __syncwarp();
-        for (uint32_t d = lane; d < 256u; d += 32u) counts[d * tiles + tile] = h[warp][d];
-    }
-    __syncthreads();
-    for (uint32_t d = threadIdx.x; d < 256u; d += blockDim.x) {
-        const uint32_t t = (h[0][d] + h[1][d]) + (h[2][d] + h[3][d]);
-        if (t != 0u) atomicAdd(totals + d, t);
-    }
-}
-
-// Exclusive scan of the digit-major counts: each row by one 256-thread CTA
-// from its digit's base (the totals of the smaller digits), 1024 entries a
-// round, four per thread.
 __device__ __forceinline__ uint32_t block_sum256(uint32_t v, uint32_t *wsum) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -335,140 +313,61 @@ __device__ __forceinline__ uint32_t block_sum256(uint32_t v, uint32_t *wsum) {
     return t;
 }
 
-__global__ void __launch_bounds__(256) k_radix_rowscan(uint32_t *counts, uint32_t tiles,
-                                                       const uint32_t *totals) {
+// sum of each CTA's 4096 buckets
+__global__ void __launch_bounds__(256) k_sort_sums(const uint32_t *counts, uint32_t *sums) {
     __shared__ uint32_t wsum[8];
-    const uint32_t d = blockIdx.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    uint32_t base = 0;
-    for (uint32_t k = tid; k < d; k += blockDim.x) base += totals[k];
-    base = block_sum256(base, wsum);
-    uint32_t *row = counts + (size_t)d * tiles;
-    for (uint32_t c0 = 0; c0 < tiles; c0 += 1024u) {
-        const uint32_t t0 = c0 + tid * 4u;
-        uint32_t x[4], run = 0;
+    const uint4 *c = reinterpret_cast<const uint4 *>(counts + (size_t)blockIdx.x * kScanItems);
+    uint32_t v = 0;
 #pragma unroll
-        for (uint32_t i = 0; i < 4u; ++i) {
-            x[i] = t0 + i < tiles ? row[t0 + i] : 0u;
-            const uint32_t c = x[i];
-            x[i] = run;                    // exclusive within the thread
-            run += c;
-        }
-        uint32_t inc = run;                // inclusive scan of thread totals in the warp
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-            if ((int)lane >= o) inc += v;
-        }
-        __syncthreads();                   // wsum of the previous round is consumed
-        if (lane == 31u) wsum[warp] = inc;
-        __syncthreads();
-        uint32_t before = 0, total = 0;
-#pragma unroll
-        for (uint32_t w = 0; w < 8u; ++w) {
-            const uint32_t s = wsum[w];
-            before += w < warp ? s : 0u;
-            total += s;
-        }
-        const uint32_t first = base + before + inc - run;
-#pragma unroll
-        for (uint32_t i = 0; i < 4u; ++i)
-            if (t0 + i < tiles) row[t0 + i] = first + x[i];
-        base += total;
+    for (uint32_t k = 0; k < kScanItems / 1024u; ++k) {
+        const uint4 q = c[threadIdx.x + 256u * k];
+        v += (q.x + q.y) + (q.z + q.w);
     }
+    v = block_sum256(v, wsum);
+    if (threadIdx.x == 0) sums[blockIdx.x] = v;
 }
 
-// Stable scatter, one 2048-item tile per CTA of eight warps; warp w owns
-// items [256 w, 256 w + 256) of the tile.
-//   1. each warp reads its slice (8 items a lane, kept in registers) and
-//      ranks every item among the slice's items of the same digit (lanes
-//      sharing a digit in a round rank in lane order);
-//   2. per digit, the counts of the warps give each warp's first rank and the
-//      digit's total; a scan over the 256 digits gives each digit's first
-//      slot in the tile;
-//   3. every item moves to its slot of the tile sorted by (digit, index), in
-//      shared memory;
-//   4. the sorted tile is written out in slot order: slot j of digit d goes
-//      to the digit's first position for this tile (the scanned counts) plus
-//      j minus the digit's first slot.  Items of one digit leave as one run,
-//      so stores coalesce instead of touching one sector per item.
-// The order is the stable one: by tile, then by index within the tile.
-constexpr uint32_t kScatterWarps = 8;
-constexpr uint32_t kSliceItems = kTileItems / kScatterWarps;   // 256 = 8 rounds of 32
-__global__ void __launch_bounds__(32 * kScatterWarps) k_radix_scatter(
-    const uint2 *in, uint32_t n, uint32_t shift, uint32_t tiles, const uint32_t *counts,
-    uint32_t *totals, uint2 *out) {
-    __shared__ __align__(16) uint2 st[kTileItems];
-    __shared__ uint32_t wrank[kScatterWarps][256];   // per warp and digit: count, then first rank
-    __shared__ uint32_t dfirst[256];                 // first slot of each digit in the tile
-    __shared__ uint32_t gbase[256];                  // first output position of each digit
-    __shared__ uint32_t wtot[kScatterWarps];
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t tile = blockIdx.x;
-    const uint32_t begin = tile * kTileItems, end = min(n, begin + kTileItems);
-    const uint32_t cnt = end - begin;
-    if (tile == 0u) totals[tid] = 0u;    // consumed by the row scan; zero for the next sort
-    for (uint32_t i = tid; i < kScatterWarps * 256u; i += blockDim.x) (&wrank[0][0])[i] = 0u;
-    __syncthreads();
-    // 1. rank within the warp's slice
-    const uint32_t s0 = warp * kSliceItems;
-    uint2 v[8];
-    uint32_t rk[8];
+// counts -> first place of each bucket, in place: 16 buckets a thread, from
+// the sums of the CTAs before
+__global__ void __launch_bounds__(256) k_sort_scan(uint32_t *counts, const uint32_t *sums) {
+    __shared__ uint32_t wsum[8];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    uint32_t base = 0;
+    for (uint32_t k = tid; k < blockIdx.x; k += 256u) base += sums[k];
+    base = block_sum256(base, wsum);
+    uint4 *c = reinterpret_cast<uint4 *>(counts + (size_t)blockIdx.x * kScanItems) + tid * 4u;
+    uint4 q[4];
+    uint32_t run = 0;
 #pragma unroll
-    for (uint32_t k = 0; k < 8u; ++k) {
-        const uint32_t i = s0 + k * 32u + lane;
-        const unsigned valid = __ballot_sync(0xFFFFFFFFu, i < cnt);
-        v[k] = make_uint2(0u, 0u);
-        rk[k] = 0u;
-        if (i < cnt) {
-            v[k] = in[begin + i];
-            const uint32_t dg = (v[k].x >> shift) & 255u;
-            const unsigned peers = __match_any_sync(valid, dg);
-            rk[k] = wrank[warp][dg] + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-            __syncwarp(valid);
-            if ((uint32_t)(__ffs(peers) - 1) == lane) wrank[warp][dg] += (uint32_t)__popc(peers);
-        }
-        __syncwarp();
+    for (int k = 0; k < 4; ++k) {
+        q[k] = c[k];
+        const uint32_t x = q[k].x, y = q[k].y, z = q[k].z, w = q[k].w;
+        q[k] = make_uint4(run, run + x, run + x + y, run + x + y + z);
+        run += (x + y) + (z + w);
     }
-    __syncthreads();
-    // 2. per digit (one thread each): warps' first ranks, the digit's total,
-    //    then an exclusive scan of the totals over the digits
-    const uint32_t d = tid;                          // blockDim.x == 256
-    uint32_t tot = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kScatterWarps; ++w) {
-        const uint32_t c = wrank[w][d];
-        wrank[w][d] = tot;
-        tot += c;
-    }
-    gbase[d] = counts[d * tiles + tile];
-    uint32_t inc = tot;
+    uint32_t inc = run;                    // inclusive scan of thread totals in the warp
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-        if ((int)lane >= o) inc += t;
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+        if ((int)lane >= o) inc += v;
     }
-    if (lane == 31u) wtot[warp] = inc;
+    __syncthreads();                       // wsum of the base is consumed
+    if (lane == 31u) wsum[warp] = inc;
     __syncthreads();
-    uint32_t before = 0;
-    for (uint32_t w = 0; w < warp; ++w) before += wtot[w];
-    dfirst[d] = before + inc - tot;
-    __syncthreads();
-    // 3. each item to its slot of the sorted tile
+    uint32_t first = base + inc - run;
 #pragma unroll
-    for (uint32_t k = 0; k < 8u; ++k) {
-        const uint32_t i = s0 + k * 32u + lane;
-        if (i < cnt) {
-            const uint32_t dg = (v[k].x >> shift) & 255u;
-            st[dfirst[dg] + wrank[warp][dg] + rk[k]] = v[k];
-        }
-    }
-    __syncthreads();
-    // 4. slot order out: runs of one digit go to consecutive positions
-    for (uint32_t j = tid; j < cnt; j += blockDim.x) {
-        const uint2 item = st[j];
-        const uint32_t dg = (item.x >> shift) & 255u;
-        out[gbase[dg] + (j - dfirst[dg])] = item;
-    }
+    for (uint32_t w = 0; w < 8u; ++w) first += w < warp ? wsum[w] : 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        c[k] = make_uint4(first + q[k].x, first + q[k].y, first + q[k].z, first + q[k].w);
+}
+
+__global__ void __launch_bounds__(256) k_sort_place(const uint2 *place, uint32_t n,
+                                                    const uint32_t *first, uint32_t *order) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint2 p = place[i];
+    order[first[p.x] + p.y] = i;
 }
 
 // order-independent fingerprint of the outputs (autotuner consistency check)
@@ -503,6 +402,14 @@ void *queue_kernel(uint32_t fl, uint32_t refill_min) {
 
 }  // namespace
 
+// key bits used for n rays: about four buckets a ray, a multiple of a CTA's
+// share at least
+static uint32_t sort_bits(size_t n) {
+    uint32_t bits = 12;
+    while (bits < kKeyBits && ((size_t)1 << bits) < 4 * n) ++bits;
+    return bits;
+}
+
 cudaError_t QueueScratch::reserve(size_t n) {
     if (!work) {
         cudaError_t e = cudaMalloc(&work, 2 * sizeof(uint32_t));
@@ -510,28 +417,28 @@ cudaError_t QueueScratch::reserve(size_t n) {
         if (e == cudaSuccess) e = cudaMalloc(&fp, sizeof(unsigned long long));
         if (e != cudaSuccess) return e;
     }
-    if (cap >= n && kv) return cudaSuccess;
-    cudaFree(kv);
-    cudaFree(kv2);
-    cudaFree(hist);
-    kv = kv2 = nullptr;
-    hist = nullptr;
+    if (cap >= n && place) return cudaSuccess;
+    cudaFree(place);
+    cudaFree(order);
+    cudaFree(counts);
+    place = nullptr;
+    order = counts = nullptr;
     cap = 0;
-    const size_t m = std::max<size_t>(n, 1);
-    const size_t tiles = (m + kTileItems - 1) / kTileItems;
-    cudaError_t e = cudaMalloc(&kv, m * sizeof(uint2));
-    if (e == cudaSuccess) e = cudaMalloc(&kv2, m * sizeof(uint2));
-    if (e == cudaSuccess) e = cudaMalloc(&hist, (tiles + kPasses) * 256 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(hist, 0, kPasses * 256 * sizeof(uint32_t));
+    const size_t m = std::max<size_t>(n, 1), buckets = (size_t)1 << sort_bits(m);
+    cudaError_t e = cudaMalloc(&place, m * sizeof(uint2));
+    if (e == cudaSuccess) e = cudaMalloc(&order, m * sizeof(uint32_t));
+    // the buckets, then the sums of kScanItems of them
+    if (e == cudaSuccess)
+        e = cudaMalloc(&counts, (buckets + buckets / kScanItems) * sizeof(uint32_t));
     if (e == cudaSuccess) cap = n;
     return e;
 }
 
 void QueueScratch::release() {
     cudaFree(work);
-    cudaFree(kv);
-    cudaFree(kv2);
-    cudaFree(hist);
+    cudaFree(place);
+    cudaFree(order);
+    cudaFree(counts);
     cudaFree(fp);
     *this = QueueScratch();
 }
@@ -541,24 +448,18 @@ cudaError_t launch_queue(const TraceArgs &ta, const VxRay *rays, size_t n, VxHit
                          cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const uint32_t nn = (uint32_t)n;
-    const uint2 *order = nullptr;
+    const uint32_t *order = nullptr;
     if (t.sort) {
-        const uint32_t tiles = (nn + kTileItems - 1) / kTileItems;
-        const unsigned tb = (tiles + 3) / 4;
-        // digit totals (256 per pass, zero between sorts), then the counts
-        uint32_t *totals = sc.hist, *counts = sc.hist + kPasses * 256u;
-        k_radix_keys<<<tiles, 256, 0, s>>>(rays, nn, ta.ro[0], ta.ro[2], sc.kv, tiles, counts,
-                                           totals);
-        uint2 *in = sc.kv, *out = sc.kv2;
-        for (uint32_t pass = 0; pass < kPasses; ++pass, totals += 256) {
-            const uint32_t shift = 8u * pass;
-            if (pass > 0) k_radix_hist<<<tb, 128, 0, s>>>(in, nn, shift, tiles, counts, totals);
-            k_radix_rowscan<<<256, 256, 0, s>>>(counts, tiles, totals);
-            k_radix_scatter<<<tiles, 32 * kScatterWarps, 0, s>>>(in, nn, shift, tiles, counts,
-                                                                 totals, out);
-            std::swap(in, out);
-        }
-        order = in;
+        const uint32_t bits = sort_bits(n), buckets = 1u << bits;
+        uint32_t *sums = sc.counts + buckets;
+        cudaError_t e = cudaMemsetAsync(sc.counts, 0, (size_t)buckets * sizeof(uint32_t), s);
+        if (e != cudaSuccess) return e;
+        k_sort_count<<<(nn + 255) / 256, 256, 0, s>>>(rays, nn, ta.ro[0], ta.ro[2],
+                                                      kKeyBits - bits, sc.counts, sc.place);
+        k_sort_sums<<<buckets / kScanItems, 256, 0, s>>>(sc.counts, sums);
+        k_sort_scan<<<buckets / kScanItems, 256, 0, s>>>(sc.counts, sums);
+        k_sort_place<<<(nn + 255) / 256, 256, 0, s>>>(sc.place, nn, sc.counts, sc.order);
+        order = sc.order;
     }
     QueueArgs q;
     q.ta = ta;
