@@ -304,6 +304,30 @@ def test_device_far_chunks():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("cx,cz", [(0, 0), (-1, 5), (63, -64), (1 << 17, -(1 << 16)),
+                                   ((1 << 18) - 1, 1 << 19), (-(1 << 19) + 1, (1 << 20) - 3)])
+def test_device_chunk_stacks_equal_oracle(cx, cz):
+    """All eight chunks over a point -- solid, surface, water and caves, all
+    air -- near the origin and where float coordinates start to skip noise
+    cells, written over a window's earlier chunks."""
+    _gpu()
+    import voxelg_b200 as vg
+    dw = vg.DeviceWorld(*DEMO)
+    dw.fill_window(7, 3, 3)
+    for seed in (SEED, 5, 0x1234_5678_0000_0009):
+        dw.gen_chunks(seed, [(cx + d, cy, cz) for d in range(4) for cy in range(8)])
+        got = dw.download()["bricks"].reshape(128, 64, 128)
+        for d in range(4):
+            for cy in range(8):
+                sx, sz = (cx + d) % 16, cz % 16
+                blk = np.ascontiguousarray(got[sz * 8:sz * 8 + 8, cy * 8:cy * 8 + 8,
+                                               sx * 8:sx * 8 + 8]).reshape(-1)
+                want = po.gen_slot_bricks(cx + d, cy, cz, seed)
+                assert np.array_equal(blk.view(np.uint8), want.view(np.uint8)), (seed, d, cy)
+    dw.close()
+
+
+@pytest.mark.gpu
 def test_frame_on_reference_world():
     """Primary and shadow rays over the reference's own demo world
     (fill_demo_terrain at seed 0xC0FFEE_F00D_BEEF): trees, leaf fringe and

@@ -13,7 +13,7 @@
 //                  and one thread per tree candidate of each distinct source
 //                  chunk (trees_for_chunk, :1537-1591), expanded into its
 //                  paint primitives (paint_tree, :1605-1710);
-//   k_gen_slot     one 256-thread CTA per storage chunk, four per SM: the
+//   k_gen_slot     one 256-thread CTA per storage chunk, three per SM: the
 //                  voxels of its columns in shared memory (ore noise from
 //                  tables of the chunk's lattice hashes), then the
 //                  primitives of the 3x3 source chunks in the reference's
@@ -33,7 +33,11 @@
 // noise hashed column by column (526 M warp instructions), all 256 threads on
 // one primitive at a time behind a barrier and the 108 tree headers read one
 // after the other; 620 us with the lattice tables, 455 us with the slabs,
-// 392 us with the chunks below ground started first (288 M).
+// 392 us with the chunks below ground started first (288 M); 355 us with a
+// tree's four levels of a slab painted at once, 350 us with two columns' noise
+// in one loop (three CTAs of 80 registers; 438 us with four of 64, which
+// spill in it), 325 us with the two columns in packed arithmetic (207 M).
+// All-air chunks only write, and caves read tables like the ores (302 M -> 275).
 // powf, cosf and sinf give the host C library's binary32 results, as the
 // reference's f32::powf / cos / sin do: vx_gmath.h's functions, corrected
 // by the exception table (Seed::lmx) on the generator's domains.
@@ -355,8 +359,8 @@ __device__ __forceinline__ void tree_voxel(uint8_t *s_mat, uint32_t dx, uint32_t
     if (cur == 0 || (cur == M_FRINGE && mat != M_FRINGE)) s_mat[v] = mat;
 }
 
-// One warp paints a primitive's voxels in the slab [zlo, zhi) of the chunk at
-// lo (any order: one primitive writes one material).
+// One warp paints a primitive's voxels in the slab [zlo, zhi = zlo + 4) of the
+// chunk at lo (any order: one primitive writes one material).
 __device__ __forceinline__ void paint_prim(uint8_t *s_mat, const int32_t lo[3], int32_t zlo,
                                            int32_t zhi, const Prim &p) {
     const uint32_t kind = p.kind_mat >> 8;
@@ -381,17 +385,28 @@ __device__ __forceinline__ void paint_prim(uint8_t *s_mat, const int32_t lo[3], 
     // without the widening.  Two rows of 16 voxels a round.
     const int32_t wide = kind == PR_SHELL ? 1 : 0, r = p.b[0], r2 = r * r;
     const int32_t ya = max(p.a[1] - r, lo[1]), yb = min(p.a[1] + r, lo[1] + kCV - 1);
-    const int32_t za = max(p.a[2] - r - wide, zlo), zb = min(p.a[2] + r + wide, zhi - 1);
-    for (int32_t z = za; z <= zb; ++z) {
-        const int32_t hz = max(abs(z - p.a[2]) - wide, 0);
-        for (int32_t y = ya + (lane >> 4); y <= yb; y += 2) {
-            const int32_t dy = y - p.a[1], rest = r2 - hz * hz - dy * dy;
-            for (int32_t dx = (lane & 15) - r - wide; dx <= r + wide; dx += 16) {
-                const int32_t hx = max(abs(dx) - wide, 0);
-                const uint32_t x = (uint32_t)(p.a[0] + dx - lo[0]);
-                if (hx * hx <= rest && x < (uint32_t)kCV)
-                    tree_voxel(s_mat, x, (uint32_t)(y - lo[1]), (uint32_t)(z - lo[2]), mat);
-            }
+    // the slab's four levels at once (they lie in one brick layer), so the
+    // reads of a row do not wait for the writes of the level before
+    int32_t hz2[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int32_t hz = max(abs(zlo + k - p.a[2]) - wide, 0);
+        hz2[k] = hz * hz;
+    }
+    for (int32_t y = ya + (lane >> 4); y <= yb; y += 2) {
+        const int32_t dy = y - p.a[1], rest_y = r2 - dy * dy;
+        for (int32_t dx = (lane & 15) - r - wide; dx <= r + wide; dx += 16) {
+            const int32_t hx = max(abs(dx) - wide, 0), rest = rest_y - hx * hx;
+            const uint32_t x = (uint32_t)(p.a[0] + dx - lo[0]);
+            if (rest < 0 || x >= (uint32_t)kCV) continue;
+            uint8_t *v = s_mat + vox(x, (uint32_t)(y - lo[1]), (uint32_t)(zlo - lo[2]));
+            uint8_t cur[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) cur[k] = v[4 * k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (hz2[k] <= rest && (cur[k] == 0 || (cur[k] == M_FRINGE && mat != M_FRINGE)))
+                    v[4 * k] = mat;
         }
     }
 }
@@ -503,7 +518,7 @@ __global__ void __launch_bounds__(256) k_gen_xz(GenPlan p, Dims d, Seed g, uint3
 }
 
 // ------------------------------------------------------------------ chunks
-constexpr int kSlotThreads = 256;   // four CTAs per SM overlap each other's barriers
+constexpr int kSlotThreads = 256;   // three CTAs per SM overlap each other's barriers
 static_assert(kTrees <= 9 * kCand && (512 % kSlotThreads) == 0, "write-out covers 512 bricks");
 
 // Job b of a plan (kGenJobInts ints, the layout of explicit plans).
@@ -527,41 +542,60 @@ __device__ __forceinline__ void job_of(const GenPlan &p, const Dims &d, uint32_t
         job[7 + k] = (cx + k % 3 - 1 - (p.ox - 1)) + (cz + k / 3 - 1 - (p.oz - 1)) * (sxn + 2);
 }
 
-// The two ore noises of stone_or_ore (voxel.rs:1906-1916) over half a chunk,
-// 16 levels at a time: the hashes of the lattice points the half can touch
-// lie in shared memory, and what depends on y alone -- the lattice row and
-// the smoothed fraction -- in a table of the chunk's 32 levels.
+// The two ore noises of stone_or_ore (voxel.rs:1906-1916) and the two of the
+// caves (:1333-1461) over half a chunk, 16 levels at a time: the
+// hashes of the lattice points the half can touch lie in shared memory, and
+// what depends on y alone -- the lattice row and the smoothed fraction -- in
+// tables of the chunk's 32 levels.
 // A voxel column by itself hashes each of its lattice cells' new corners (36
-// and 74 hashes per column for the two frequencies, 1,024 columns); a half
-// has 847 and 4,400 lattice points.
+// and 74 hashes per column for the ore frequencies, 1,024 columns); a half
+// has 847 and 4,400 lattice points, and 64 and 108 of the caves'.
 constexpr float kOreF1 = 0.27f, kOreF2 = 0.55f;
+constexpr float kCaveF1 = 0.045f, kCaveF2 = 0.110f, kCaveY1 = 0.085f, kCaveY2 = 0.060f;
 constexpr int kHalf = 16;
-constexpr int kN1 = 11, kY1 = 7, kN2 = 20, kY2 = 11;   // points: 31 f + 2 and 15 f + 2, rounded up
-struct OreLevel {
-    float yf, yg;       // smoothed fraction and 1 - it
-    int32_t yi;         // lattice row
-    int32_t pad;
+// points: 31 f + 2 in x and z, 15 f + 2 in y, rounded up
+constexpr int kN1 = 11, kY1 = 7, kN2 = 20, kY2 = 11, kN3 = 4, kY3 = 4, kN4 = 6, kY4 = 3;
+struct __align__(16) NoiseLevel {
+    float yf, yf2, yg, yg2;     // smoothed fraction and 1 - it, twice each
 };
 struct SlotShared {
     uint8_t mat[kCV * kCV * kCV];
-    float t1[kY1 * kN1 * kN1], t2[kY2 * kN2 * kN2];
-    OreLevel l1[kCV], l2[kCV];
+    float t1[kY1 * kN1 * kN1], t2[kY2 * kN2 * kN2], t3[kY3 * kN3 * kN3], t4[kY4 * kN4 * kN4];
+    NoiseLevel l[4][kCV];
+    int32_t row[4][kCV];            // lattice row of each level
+    float one[2];                   // 1
+    uint32_t step[4];               // bit y: its row is the one after level y - 1's
     int32_t job[kGenJobInts];
-    uint8_t uni[512], solid[512];   // per brick: uniform byte, any voxel
+    int32_t x0[4], z0[4];           // first cells of the tables
+    // per brick: uniform byte, any voxel (once the tables are done with)
+    __device__ uint8_t *uni() { return reinterpret_cast<uint8_t *>(t2); }
+    __device__ uint8_t *solid() { return uni() + 512; }
 };
+static_assert(3 * (sizeof(SlotShared) + 1024) <= 228 * 1024, "three CTAs per SM");
 // one noise of a column, read from the lattice table: value_noise_3d's
 // operations on the same hashes
 template <int N>
-struct OreColumn {
-    const float *t;     // the column's lattice cell in the table, row 0
-    float xf, xg, zf, zg;
+struct TableColumn {
+    int32_t at;         // the column's lattice cell in lattice row 0 of the table
+    float xf, zf, zg;
     float a, b, c, d;
     int32_t yi;
-    __device__ __forceinline__ float lerp(const float *q) const { return q[0] * xg + q[1] * xf; }
-    __device__ __forceinline__ float eval(const OreLevel &l, int32_t y_first) {
-        if (l.yi != yi) {
-            const float *q = t + (l.yi - y_first) * (N * N);
-            if (l.yi == yi + 1) {
+    // x and z times the frequency; the table's first cell
+    __device__ __forceinline__ void init(float x, float z, int32_t x0, int32_t y0, int32_t z0) {
+        const int32_t xi = noise::floor_i(x), zi = noise::floor_i(z);
+        xf = noise::smooth(x - (float)xi);
+        zf = noise::smooth(z - (float)zi);
+        zg = 1.0f - zf;
+        at = ((zi - z0) - y0 * N) * N + (xi - x0);
+        yi = INT32_MIN;
+    }
+    __device__ __forceinline__ float lerp(const float *q) const {
+        return q[0] * (1.0f - xf) + q[1] * xf;
+    }
+    __device__ __forceinline__ float eval(const float *t, const NoiseLevel &l, int32_t row) {
+        if (row != yi) {
+            const float *q = t + (at + row * (N * N));
+            if (row == yi + 1) {
                 a = b;
                 c = d;
             } else {
@@ -570,15 +604,81 @@ struct OreColumn {
             }
             b = lerp(q + N * N);
             d = lerp(q + N * N + N);
-            yi = l.yi;
+            yi = row;
         }
         const float ab = a * l.yg + b * l.yf;
         const float cd = c * l.yg + d * l.yf;
         return ab * zg + cd * zf;
     }
 };
-__device__ __forceinline__ uint8_t ore_of(float n1, float n2, int32_t depth) {
-    const float combined = n1 + n2 * 0.30f;
+// Two columns at once, of one x and two z: the same operations, two to an
+// instruction (each half of a float pair rounds by itself).  Their y levels go
+// up one by one from the half's first.
+// A pair's mul and add came out contracted into one rounding (one ore voxel of
+// a 512x256x512 window fell on the other side of its threshold), so sums are
+// a * one + b, with a one that the compiler does not know: a's product is
+// rounded before it is multiplied, and times one is exact.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pair(float lo, float hi) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpair(f2 v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b, f2 one) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(one), "l"(b));
+    return r;
+}
+template <int N>
+struct TablePair {
+    const float *q0, *q1;   // the columns' cells in the upper lattice row
+    float xf, xg;
+    f2 zf, zg, a, b, c, d;
+    __device__ __forceinline__ f2 lerp(int o, f2 one) const {
+        return add2(mul2(pair(q0[o], q1[o]), pair(xg, xg)),
+                    mul2(pair(q0[o + 1], q1[o + 1]), pair(xf, xf)), one);
+    }
+    __device__ __forceinline__ void init(const float *t, float x, float za, float zb, int32_t x0,
+                                         int32_t z0, f2 one) {
+        const int32_t xi = noise::floor_i(x), zi = noise::floor_i(za), zj = noise::floor_i(zb);
+        xf = noise::smooth(x - (float)xi);
+        xg = 1.0f - xf;
+        const float fa = noise::smooth(za - (float)zi), fb = noise::smooth(zb - (float)zj);
+        zf = pair(fa, fb);
+        zg = pair(1.0f - fa, 1.0f - fb);
+        q0 = t + (zi - z0) * N + (xi - x0);
+        q1 = t + (zj - z0) * N + (xi - x0);
+        a = lerp(0, one);
+        c = lerp(N, one);
+        q0 += N * N;
+        q1 += N * N;
+        b = lerp(0, one);
+        d = lerp(N, one);
+    }
+    __device__ __forceinline__ void step(f2 one) {
+        q0 += N * N;
+        q1 += N * N;
+        a = b;
+        c = d;
+        b = lerp(0, one);
+        d = lerp(N, one);
+    }
+    __device__ __forceinline__ f2 eval(const NoiseLevel &l, f2 one) const {
+        const f2 yf = pair(l.yf, l.yf2), yg = pair(l.yg, l.yg2);
+        const f2 ab = add2(mul2(a, yg), mul2(b, yf), one);
+        const f2 cd = add2(mul2(c, yg), mul2(d, yf), one);
+        return add2(mul2(ab, zg), mul2(cd, zf), one);
+    }
+};
+__device__ __forceinline__ uint8_t ore_of(float combined, int32_t depth) {
     if (depth > 30 && combined > 0.50f) return M_DIAMOND;
     if (depth > 20 && combined > 0.36f) return M_GOLD;
     if (depth > 10 && combined > 0.24f) return M_IRON;
@@ -586,7 +686,65 @@ __device__ __forceinline__ uint8_t ore_of(float n1, float n2, int32_t depth) {
     return M_STONE;
 }
 
-__global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPlan pl) {
+// The two kinds of column that few chunks have are calls, so their noises'
+// registers are not the kernel's (inlined: 334 us against 325 for an 8 x 3
+// chunk step of a 2048x2048 window).
+//
+// Levels [y, end) of stone and ore with caves below `seal`, from the tables.
+__device__ __noinline__ void cave_column(SlotShared &sh, float wx, float wz, uint32_t dx,
+                                         uint32_t dz, int32_t y0, int half, int32_t end,
+                                         int32_t seal, int32_t h) {
+    const int first = half * kHalf;
+    TableColumn<kN1> o1;
+    TableColumn<kN2> o2;
+    TableColumn<kN3> c1;
+    TableColumn<kN4> c2;
+    o1.init(wx * kOreF1, wz * kOreF1, sh.x0[0], sh.row[0][first], sh.z0[0]);
+    o2.init(wx * kOreF2, wz * kOreF2, sh.x0[1], sh.row[1][first], sh.z0[1]);
+    c1.init(wx * kCaveF1, wz * kCaveF1, sh.x0[2], sh.row[2][first], sh.z0[2]);
+    c2.init(wx * kCaveF2, wz * kCaveF2, sh.x0[3], sh.row[3][first], sh.z0[3]);
+    for (int32_t y = y0 + first; y < end; ++y) {
+        const int l = y - y0;
+        if (y < seal && y > 4) {
+            const float cn = c1.eval(sh.t3, sh.l[2][l], sh.row[2][l]);
+            const float cn2 = c2.eval(sh.t4, sh.l[3][l], sh.row[3][l]);
+            if ((cn + cn2 * 0.6f) > 0.30f) continue;
+        }
+        const float n1 = o1.eval(sh.t1, sh.l[0][l], sh.row[0][l]);
+        const float n2 = o2.eval(sh.t2, sh.l[1][l], sh.row[1][l]);
+        sh.mat[vox(dx, (uint32_t)l, dz)] = ore_of(n1 + n2 * 0.30f, h - y);
+    }
+}
+
+// Levels [y, end) up to the surface of a column beyond the tables.
+__device__ __noinline__ void direct_column(uint8_t *s_mat, float wx, float wz, uint32_t dx,
+                                           uint32_t dz, int32_t y0, int32_t y, int32_t end,
+                                           int32_t seal, int32_t h, int biome) {
+    noise::ColumnNoise3 ore1, ore2, cave1, cave2;
+    ore1.init(wx * kOreF1, wz * kOreF1);
+    ore2.init(wx * kOreF2, wz * kOreF2);
+    cave1.init(wx * kCaveF1, wz * kCaveF1);
+    cave2.init(wx * kCaveF2, wz * kCaveF2);
+    for (; y < end && y <= h; ++y) {
+        if (!(y >= seal) && y > 4 && y + 3 < h) {
+            const float cn = cave1.eval((float)y * kCaveY1);
+            const float cn2 = cave2.eval((float)y * kCaveY2);
+            if ((cn + cn2 * 0.6f) > 0.30f) continue;
+        }
+        uint8_t mat;
+        if (y >= h) {
+            mat = top_block(biome, (uint32_t)h);
+        } else if (y + 4 >= h) {
+            mat = subsoil(biome);
+        } else {
+            const float n1 = ore1.eval((float)y * kOreF1), n2 = ore2.eval((float)y * kOreF2);
+            mat = ore_of(n1 + n2 * 0.30f, h - y);
+        }
+        s_mat[vox(dx, (uint32_t)(y - y0), dz)] = mat;
+    }
+}
+
+__global__ void __launch_bounds__(kSlotThreads, 3) k_gen_slot(DevWorld w, GenPlan pl) {
     extern __shared__ __align__(16) uint8_t s_raw[];
     SlotShared &sh = *reinterpret_cast<SlotShared *>(s_raw);
     uint8_t *s_mat = sh.mat;
@@ -600,13 +758,54 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
     const uint32_t tid = threadIdx.x;
     const Prim *prims = reinterpret_cast<const Prim *>(pl.prims);
 
-    uint4 *z4 = reinterpret_cast<uint4 *>(s_mat);
-    for (uint32_t i = tid; i < (uint32_t)(kCV * kCV * kCV / 16); i += kSlotThreads)
-        z4[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
     const int32_t *job = s_job;
     const int32_t lo[3] = {job[0] * kCV, job[1] * kCV, job[2] * kCV};
     const uint32_t *colw = pl.colw + (size_t)job[6] * (kCV * kCV);
+    const uint32_t sbx = (uint32_t)job[3] * 8u, sby = (uint32_t)job[4] * 8u,
+                   sbz = (uint32_t)job[5] * 8u;
+    int32_t h_max = -1;
+    {
+        bool any = false;               // can anything be in this chunk?
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t word = __ldg(colw + tid + kSlotThreads * i);
+            const int32_t h = (int32_t)(word & 0xFFu);
+            h_max = max(h_max, h);
+            // two levels of decoration over the column, or its water
+            any = any || max(h + 2, (word >> 8) & 1u ? kSea : 0) >= lo[1];
+        }
+        if (tid < (uint32_t)kTrees) {
+            const int32_t hd = __ldg(pl.hdr + (size_t)job[7 + tid / kCand] * kCand + tid % kCand);
+            any = any || ((hd & 0xFF) != 0 && (hd >> 18) <= lo[1] + kCV && (hd >> 18) + 22 >= lo[1]);
+        }
+        if (__syncthreads_or(any) == 0) {
+            // all air (three quarters of the chunks): rows of eight bricks
+            for (uint32_t i = tid; i < 2048u; i += kSlotThreads) {
+                const uint32_t r = i >> 5;
+                const size_t gbi = sbx + (sby + (r & 7u)) * (size_t)w.d.bx +
+                                   (sbz + (r >> 3)) * (size_t)(w.d.bx * w.d.by);
+                reinterpret_cast<uint4 *>(w.mat + gbi * 64u)[i & 31u] = make_uint4(0, 0, 0, 0);
+            }
+            for (uint32_t b = tid; b < 512u; b += kSlotThreads) {
+                const size_t gbi = (sbx + (b & 7u)) + (sby + ((b >> 3) & 7u)) * (size_t)w.d.bx +
+                                   (sbz + (b >> 6)) * (size_t)(w.d.bx * w.d.by);
+                w.occ[gbi] = 0ull;
+                w.brick_uniform[gbi] = 0;
+            }
+            if (tid < 8u) {
+                const int64_t ti = (int64_t)(job[3] * 2 + (int32_t)(tid & 1u)) +
+                                   (int64_t)(job[4] * 2 + (int32_t)((tid >> 1) & 1u)) * w.d.tx +
+                                   (int64_t)(job[5] * 2 + (int32_t)(tid >> 2)) * w.d.tx * w.d.ty;
+                w.tile_mask[ti] = 0ull;
+                w.tile_uniform[ti] = 0;
+            }
+            return;
+        }
+    }
+    uint4 *zero = reinterpret_cast<uint4 *>(s_mat);
+    for (uint32_t i = tid; i < (uint32_t)(kCV * kCV * kCV / 16); i += kSlotThreads)
+        zero[i] = make_uint4(0, 0, 0, 0);
 
     // ---- the columns (dx, dz), voxel.rs:1333-1461
     // Thread: dx = its lane, dz = its warp + 8 i.
@@ -616,97 +815,121 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
     const float wx = (float)wxi;
     // x and z lattice cells; a chunk so far out that binary32 coordinates
     // skip cells does not fit the tables and evaluates its noise directly
-    const int32_t x1 = noise::floor_i((float)lo[0] * kOreF1), x2 = noise::floor_i((float)lo[0] * kOreF2);
-    const int32_t z1 = noise::floor_i((float)lo[2] * kOreF1), z2 = noise::floor_i((float)lo[2] * kOreF2);
+    const float xb = (float)lo[0], zb = (float)lo[2];
+    const int32_t x1 = noise::floor_i(xb * kOreF1), x2 = noise::floor_i(xb * kOreF2);
+    const int32_t z1 = noise::floor_i(zb * kOreF1), z2 = noise::floor_i(zb * kOreF2);
+    const int32_t x3 = noise::floor_i(xb * kCaveF1), x4 = noise::floor_i(xb * kCaveF2);
+    const int32_t z3 = noise::floor_i(zb * kCaveF1), z4 = noise::floor_i(zb * kCaveF2);
     const float xe = (float)(lo[0] + kCV - 1), ze = (float)(lo[2] + kCV - 1);
     const bool tables = noise::floor_i(xe * kOreF1) - x1 + 2 <= kN1 &&
                         noise::floor_i(ze * kOreF1) - z1 + 2 <= kN1 &&
                         noise::floor_i(xe * kOreF2) - x2 + 2 <= kN2 &&
-                        noise::floor_i(ze * kOreF2) - z2 + 2 <= kN2;
-    if (tid < (uint32_t)kCV) {
-        const float fy = (float)(y0 + (int32_t)tid);
-        const float p1 = fy * kOreF1, p2 = fy * kOreF2;
-        const int32_t i1 = noise::floor_i(p1), i2 = noise::floor_i(p2);
-        const float f1 = noise::smooth(p1 - (float)i1), f2 = noise::smooth(p2 - (float)i2);
-        sh.l1[tid] = OreLevel{f1, 1.0f - f1, i1, 0};
-        sh.l2[tid] = OreLevel{f2, 1.0f - f2, i2, 0};
+                        noise::floor_i(ze * kOreF2) - z2 + 2 <= kN2 &&
+                        noise::floor_i(xe * kCaveF1) - x3 + 2 <= kN3 &&
+                        noise::floor_i(ze * kCaveF1) - z3 + 2 <= kN3 &&
+                        noise::floor_i(xe * kCaveF2) - x4 + 2 <= kN4 &&
+                        noise::floor_i(ze * kCaveF2) - z4 + 2 <= kN4;
+    if (tid == 0) {
+        sh.one[0] = sh.one[1] = 1.0f;
+        sh.x0[0] = x1; sh.x0[1] = x2; sh.x0[2] = x3; sh.x0[3] = x4;
+        sh.z0[0] = z1; sh.z0[1] = z2; sh.z0[2] = z3; sh.z0[3] = z4;
     }
-    uint32_t words[4];
-    int32_t h_max = -1;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        words[i] = colw[tid + (uint32_t)(kSlotThreads * i)];
-        h_max = max(h_max, (int32_t)(words[i] & 0xFFu));
+    if (tid < 4u * kCV) {
+        const uint32_t q = tid >> 5, l = tid & 31u;     // noise, level
+        const float f = q == 0u ? kOreF1 : (q == 1u ? kOreF2 : (q == 2u ? kCaveY1 : kCaveY2));
+        const float py = (float)(y0 + (int32_t)l) * f;
+        const int32_t yi = noise::floor_i(py);
+        const float yf = noise::smooth(py - (float)yi);
+        sh.l[q][l] = NoiseLevel{yf, yf, 1.0f - yf, 1.0f - yf};
+        sh.row[q][l] = yi;
+        const int32_t below = __shfl_up_sync(0xFFFFFFFFu, yi, 1);
+        const uint32_t step = __ballot_sync(0xFFFFFFFFu, l != 0u && yi != below);
+        if (l == 0u) sh.step[q] = step;
     }
     for (int half = 0; half < kCV / kHalf; ++half) {
         const int32_t ylo = y0 + half * kHalf, yhi = ylo + kHalf;
         // any voxel of stone or ore (y + 4 < h) in this half?
         const bool ore = __syncthreads_or(ylo + 4 < h_max) != 0 && tables;
-        const int32_t r1 = sh.l1[half * kHalf].yi, r2 = sh.l2[half * kHalf].yi;
+        const int32_t r1 = sh.row[0][half * kHalf], r2 = sh.row[1][half * kHalf];
+        const int32_t r3 = sh.row[2][half * kHalf], r4 = sh.row[3][half * kHalf];
         if (ore) {
             for (uint32_t i = tid; i < (uint32_t)(kY1 * kN1 * kN1); i += kSlotThreads)
-                sh.t1[i] = hash3(x1 + (int32_t)(i % kN1), r1 + (int32_t)(i / (kN1 * kN1)),
-                                 z1 + (int32_t)((i / kN1) % kN1));
+                sh.t1[i] = hash3(sh.x0[0] + (int32_t)(i % kN1), r1 + (int32_t)(i / (kN1 * kN1)),
+                                 sh.z0[0] + (int32_t)((i / kN1) % kN1));
             for (uint32_t i = tid; i < (uint32_t)(kY2 * kN2 * kN2); i += kSlotThreads)
-                sh.t2[i] = hash3(x2 + (int32_t)(i % kN2), r2 + (int32_t)(i / (kN2 * kN2)),
-                                 z2 + (int32_t)((i / kN2) % kN2));
+                sh.t2[i] = hash3(sh.x0[1] + (int32_t)(i % kN2), r2 + (int32_t)(i / (kN2 * kN2)),
+                                 sh.z0[1] + (int32_t)((i / kN2) % kN2));
+            for (uint32_t i = tid; i < (uint32_t)(kY3 * kN3 * kN3); i += kSlotThreads)
+                sh.t3[i] = hash3(sh.x0[2] + (int32_t)(i % kN3), r3 + (int32_t)(i / (kN3 * kN3)),
+                                 sh.z0[2] + (int32_t)((i / kN3) % kN3));
+            for (uint32_t i = tid; i < (uint32_t)(kY4 * kN4 * kN4); i += kSlotThreads)
+                sh.t4[i] = hash3(sh.x0[3] + (int32_t)(i % kN4), r4 + (int32_t)(i / (kN4 * kN4)),
+                                 sh.z0[3] + (int32_t)((i / kN4) % kN4));
             __syncthreads();
         }
+        bool caves = false;             // any in the warp's pair of rows of columns?
         for (int i = 0; i < 4; ++i) {
-            const uint32_t word = words[i];
+            const uint32_t word = __ldg(colw + tid + kSlotThreads * i);
             const int32_t h = (int32_t)(word & 0xFFu);
-            const uint32_t hu = (uint32_t)h;
             const int32_t water_top = (word >> 8) & 1u ? kSea : 0;
             const int col_top = max(h, water_top);
-            if (col_top < ylo) continue;
-            const int biome = (int)((word >> 9) & 7u);
+            // caves only under water, below its seal
+            const int32_t seal = water_top > h ? h - 5 : INT32_MIN;
             const uint32_t dx = lane, dz = warp + 8u * (uint32_t)i;
             const float wz = (float)(lo[2] + (int32_t)dz);
-            const int32_t ye = min(yhi, kWorldY);
-            int32_t y = ylo;
-            // below the subsoil, caves only under water (their seal): stone and ore
-            const int32_t seal = water_top > h ? h - 5 : INT32_MIN;
-            const int32_t ore_end = min(ye, h - 4);      // y + 4 < h
-            if (ore && seal == INT32_MIN) {
-                OreColumn<kN1> o1;
-                OreColumn<kN2> o2;
-                const float px1 = wx * kOreF1, pz1 = wz * kOreF1, px2 = wx * kOreF2, pz2 = wz * kOreF2;
-                const int32_t xi1 = noise::floor_i(px1), zi1 = noise::floor_i(pz1);
-                const int32_t xi2 = noise::floor_i(px2), zi2 = noise::floor_i(pz2);
-                o1.xf = noise::smooth(px1 - (float)xi1); o1.xg = 1.0f - o1.xf;
-                o1.zf = noise::smooth(pz1 - (float)zi1); o1.zg = 1.0f - o1.zf;
-                o2.xf = noise::smooth(px2 - (float)xi2); o2.xg = 1.0f - o2.xf;
-                o2.zf = noise::smooth(pz2 - (float)zi2); o2.zg = 1.0f - o2.zf;
-                o1.t = sh.t1 + (zi1 - z1) * kN1 + (xi1 - x1);
-                o2.t = sh.t2 + (zi2 - z2) * kN2 + (xi2 - x2);
-                o1.yi = o2.yi = INT32_MIN;
-                for (; y < ore_end; ++y) {
-                    const float n1 = o1.eval(sh.l1[y - y0], r1);
-                    const float n2 = o2.eval(sh.l2[y - y0], r2);
-                    s_mat[vox(dx, (uint32_t)(y - y0), dz)] = ore_of(n1, n2, h - y);
+            // below the subsoil (y + 4 < h) stone and ore: without caves two
+            // columns at once, dz and dz + 8
+            if ((i & 1) == 0 && ore) {
+                const uint32_t next = __ldg(colw + tid + kSlotThreads * (i + 1));
+                const int32_t hn = (int32_t)(next & 0xFFu);
+                const int32_t sn = ((next >> 8) & 1u) && kSea > hn ? hn - 5 : INT32_MIN;
+                caves = __any_sync(0xFFFFFFFFu, ylo < max(seal, sn));
+                const int32_t ea = min(yhi, h - 4), eb = min(yhi, hn - 4), e = max(ea, eb);
+                if (!caves && ylo < e) {
+                    TablePair<kN1> o1;
+                    TablePair<kN2> o2;
+                    const f2 one = pair(sh.one[0], sh.one[1]), third = pair(0.30f, 0.30f);
+                    const float wn = (float)(lo[2] + (int32_t)dz + 8);
+                    o1.init(sh.t1, wx * kOreF1, wz * kOreF1, wn * kOreF1, sh.x0[0], sh.z0[0],
+                            one);
+                    o2.init(sh.t2, wx * kOreF2, wz * kOreF2, wn * kOreF2, sh.x0[1], sh.z0[1],
+                            one);
+                    // bit 0: the next level's
+                    uint32_t s1 = sh.step[0] >> (half * kHalf), s2 = sh.step[1] >> (half * kHalf);
+                    uint8_t *v = s_mat + vox(dx, (uint32_t)(half * kHalf), dz);
+                    for (int32_t y = ylo;;) {
+                        const f2 n = add2(mul2(o2.eval(sh.l[1][y - y0], one), third),
+                                          o1.eval(sh.l[0][y - y0], one), one);
+                        float na, nb;
+                        unpair(n, na, nb);
+                        // 8 levels of z on: two brick layers
+                        if (y < ea) v[0] = ore_of(na, h - y);
+                        if (y < eb) v[2 * 64 * 64] = ore_of(nb, hn - y);
+                        if (++y >= e) break;
+                        v += (y & 3) != 0 ? 16 : 8 * 64 - 48;
+                        s1 >>= 1;
+                        s2 >>= 1;
+                        if (s1 & 1u) o1.step(one);
+                        if (s2 & 1u) o2.step(one);
+                    }
                 }
             }
-            if (y < ye && y <= h) {
-                // the rest of the column: surface and subsoil, and whole
-                // columns with caves or beyond the tables
-                noise::ColumnNoise3 ore1, ore2, cave1, cave2;
-                ore1.init(wx * kOreF1, wz * kOreF1);
-                ore2.init(wx * kOreF2, wz * kOreF2);
-                cave1.init(wx * 0.045f, wz * 0.045f);
-                cave2.init(wx * 0.110f, wz * 0.110f);
-                for (; y < ye; ++y) {
-                    if (y > h) break;
-                    if (!(y >= seal) && y > 4 && y + 3 < h) {
-                        const float cn = cave1.eval((float)y * 0.085f);
-                        const float cn2 = cave2.eval((float)y * 0.060f);
-                        if ((cn + cn2 * 0.6f) > 0.30f) continue;
-                    }
-                    uint8_t mat;
-                    if ((uint32_t)y >= hu) mat = top_block(biome, hu);
-                    else if ((uint32_t)y + 4u >= hu) mat = subsoil(biome);
-                    else mat = ore_of(ore1.eval((float)y * kOreF1), ore2.eval((float)y * kOreF2), h - y);
-                    s_mat[vox(dx, (uint32_t)(y - y0), dz)] = mat;
-                }
+            if (col_top < ylo) continue;
+            const int biome = (int)((word >> 9) & 7u);
+            const int32_t ye = min(yhi, kWorldY);
+            int32_t y = ylo;
+            if (ore) {
+                const int32_t ore_end = min(ye, h - 4);
+                if (caves) cave_column(sh, wx, wz, dx, dz, y0, half, ore_end, seal, h);
+                y = max(ylo, ore_end);
+            }
+            if (tables) {
+                // subsoil and surface (y + 4 >= h: neither ore nor caves)
+                const uint8_t sub = subsoil(biome), top = top_block(biome, (uint32_t)h);
+                for (; y < ye && y <= h; ++y)
+                    s_mat[vox(dx, (uint32_t)(y - y0), dz)] = y >= h ? top : sub;
+            } else if (y < ye && y <= h) {
+                direct_column(s_mat, wx, wz, dx, dz, y0, y, ye, seal, h, biome);
             }
             if (water_top > h) {
                 const int32_t fb = max(h + 1, ylo), fe = min(water_top, yhi - 1);
@@ -719,7 +942,7 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
     // surface decoration over the finished columns
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const uint32_t word = words[i];
+        const uint32_t word = __ldg(colw + tid + kSlotThreads * i);
         const uint32_t dec = (word >> 12) & 63u, dx = lane, dz = warp + 8u * (uint32_t)i;
         const int32_t dec_y = (int32_t)(word & 0xFFu) + 1;
         // a column that ends below the chunk decorates nothing in it
@@ -792,8 +1015,6 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
     __syncthreads();
 
     // ---- bricks out: material rows, occupancy words, uniform bytes
-    const uint32_t sbx = (uint32_t)job[3] * 8u, sby = (uint32_t)job[4] * 8u,
-                   sbz = (uint32_t)job[5] * 8u;
     for (uint32_t b = tid; b < 512u; b += kSlotThreads) {
         const uint32_t gbi = (sbx + (b & 7u)) + (sby + ((b >> 3) & 7u)) * (uint32_t)w.d.bx +
                              (sbz + (b >> 6)) * (uint32_t)(w.d.bx * w.d.by);
@@ -810,16 +1031,16 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 same = same && qs[m] == rep;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if ((qs[m] >> (8 * j)) & 0xFFu) occ |= 1ull << (16 * q4 + 4 * m + j);
+                // top bit of each byte that is not 0, the four bits side by side
+                const uint32_t nz = (((qs[m] & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | qs[m]) & 0x80808080u;
+                occ |= (uint64_t)(((nz >> 7) * 0x10204080u) >> 28) << (16 * q4 + 4 * m);
             }
         }
         w.occ[gbi] = occ;
         const uint8_t u = (occ == ~0ull && same) ? (uint8_t)m0 : (uint8_t)0;
         w.brick_uniform[gbi] = u;
-        sh.uni[b] = u;
-        sh.solid[b] = occ != 0ull ? 1u : 0u;
+        sh.uni()[b] = u;
+        sh.solid()[b] = occ != 0ull ? 1u : 0u;
     }
     __syncthreads();
     // the chunk's eight tiles, one warp each (tile word and LUT,
@@ -832,8 +1053,8 @@ __global__ void __launch_bounds__(kSlotThreads, 4) k_gen_slot(DevWorld w, GenPla
             const uint32_t c = lane + 32u * (uint32_t)q;   // child bit x + z*4 + y*16
             const uint32_t b = (tx * 4u + (c & 3u)) + (ty * 4u + (c >> 4)) * 8u +
                                (tz * 4u + ((c >> 2) & 3u)) * 64u;
-            u[q] = sh.uni[b];
-            sol[q] = sh.solid[b];
+            u[q] = sh.uni()[b];
+            sol[q] = sh.solid()[b];
         }
         const uint32_t m_lo = __ballot_sync(0xFFFFFFFFu, sol[0] != 0u);
         const uint32_t m_hi = __ballot_sync(0xFFFFFFFFu, sol[1] != 0u);
