@@ -593,10 +593,12 @@ __device__ __forceinline__ int walk_step(const DevWorld &w, const Geo &g, const 
 // the rest of a 1080p frame.
 //
 // Right after a skip the state is a function of the voxel and the crossed
-// axis: t_max is formed from the voxel, t from t_max and the axis
-// (KIND_NO_WATER keeps an older t, which then only a step changes, to a value
-// it had a cycle ago).  seen_key is that voxel and axis, one to one, and 0
-// when the state is not of that form, so two equal keys are one state.
+// axis: t_max is formed from the voxel, t from t_max and the axis.  seen_key
+// is that voxel and axis, one to one, and 0 when the state is not of that
+// form, so two equal keys are one state.  KIND_NO_WATER keeps an older t, which
+// only a step changes, and its key leaves t out: the moves do not read it, and
+// between two equal keys every t that the moves set has been held against tmax
+// but the one now in the state, which walk_to_end looks at itself.
 struct SeenKey {
     uint32_t lo, hi;      // hi == 0: none
 };
@@ -640,7 +642,7 @@ __device__ __forceinline__ int walk_to_end(const DevWorld &w, const Geo &g, cons
         }
         if (STATS || r != WALK_CAP || k.iters >= cap) break;
         const SeenKey now = seen_key(k, KNOWN >= 0 ? KNOWN == (int)KIND_NO_WATER : k.kind == KIND_NO_WATER);
-        if (now.hi != 0u && now.lo == seen.lo && now.hi == seen.hi) {
+        if (now.hi != 0u && now.lo == seen.lo && now.hi == seen.hi && !(k.t_cur > k.tmax)) {
             k.iters = cap;
             break;
         }
