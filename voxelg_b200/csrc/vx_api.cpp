@@ -52,7 +52,6 @@ struct VxWorld {
         VxPickHit out;
         int32_t hit;
         uint32_t fault;               // DevWorld::fault (kFaultBeamCopyLost)
-        uint32_t masks_bad;           // answer of launch_masks_hold
     };
     PickBox *pick = nullptr;          // host address
     PickBox *pick_dev = nullptr;      // device address of the same block
@@ -115,8 +114,13 @@ struct VxWorld {
     // every brick with a solid voxel is under set mask bits: so by
     // construction wherever the library builds the masks (updates of part of
     // them keep it), checked where the caller uploads them.  Batched picking
-    // skips by the masks then, as raycast() itself does not read them.
+    // skips by the masks then, as raycast() itself does not read them.  The
+    // host's flag picks the faster kernel; the device's word (d_masks[0],
+    // nonzero where the masks may not hold) is what the kernel goes by, so a
+    // batch that was captured in a graph or waits on another stream meets the
+    // world as it then is.  d_masks[1] is the check's own.
     std::atomic<bool> masks_hold{true};
+    uint32_t *d_masks = nullptr;
     bool tiles_built = true;         // tile words and LUT bytes are the library's, for every tile
     uint64_t df_gen = 0;
     float *lrn_depth = nullptr;      // per-tile proven depths of learned frames without a proposal
@@ -197,6 +201,13 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 constexpr uint32_t kSyncBands = 6;
 constexpr uint32_t kAsyncBands = 1;
 
+// The device's word after launches that rebuilt every mask (a world whose masks
+// hold keeps it as it is).
+cudaError_t masks_rebuilt(VxWorld *w) {
+    return w->masks_hold ? cudaSuccess
+                         : cudaMemsetAsync(w->d_masks, 0, sizeof(uint32_t), w->stream);
+}
+
 int use_device(VxWorld *w) {
     VX_CK(cudaSetDevice(w->device));
     return VX_OK;
@@ -231,6 +242,7 @@ void free_world(VxWorld *w) {
     cudaFree(w->sh);
     if (w->pick) cudaFreeHost(w->pick);
     cudaFree(w->d_work);
+    cudaFree(w->d_masks);
     cudaFree(w->d_gate_idx);
     cudaFree(w->pick_buf);
     for (auto &e : w->pick_ev)
@@ -469,6 +481,8 @@ int vx_world_create(const VxWorldDesc *desc, VxWorld **out) {
     VX_CKW(cudaMalloc(&w->d_stats, 4 * sizeof(unsigned long long)));
     VX_CKW(cudaMalloc(&w->d_work, 2 * sizeof(uint32_t)));
     VX_CKW(cudaMemsetAsync(w->d_work, 0, 2 * sizeof(uint32_t), w->stream));
+    VX_CKW(cudaMalloc(&w->d_masks, 2 * sizeof(uint32_t)));
+    VX_CKW(cudaMemsetAsync(w->d_masks, 0, 2 * sizeof(uint32_t), w->stream));
     VX_CKW(cudaHostAlloc(reinterpret_cast<void **>(&w->pick), sizeof(VxWorld::PickBox),
                          cudaHostAllocMapped));
     VX_CKW(cudaHostGetDevicePointer(reinterpret_cast<void **>(&w->pick_dev), w->pick, 0));
@@ -536,6 +550,8 @@ int vx_world_upload(VxWorld *w, const VxBrick *bricks, const uint64_t *tile_mask
     forget_generated(w);
     w->masks_hold = false;
     w->tiles_built = false;
+    VX_CK(cudaMemsetAsync(w->d_masks, 0xFF, sizeof(uint32_t), w->stream));
+    VX_CK(cudaMemsetAsync(w->d_masks + 1, 0, sizeof(uint32_t), w->stream));
     const vx::Dims &d = w->dw.d;
     const size_t chunk = (size_t)1 << 20;  // bricks per staging round (72 MiB)
     rc = ensure(&w->d_bricks, &w->bricks_cap, std::min<size_t>(chunk, (size_t)d.n_bricks));
@@ -553,10 +569,14 @@ int vx_world_upload(VxWorld *w, const VxBrick *bricks, const uint64_t *tile_mask
     VX_CK(cudaMemcpyAsync(w->dw.tile_uniform, tile_uniform, d.n_tiles, cudaMemcpyHostToDevice, w->stream));
     vx::world_masks_changed(w);
     VX_CK(vx::launch_tile_meta(w->dw, w->stream));
-    w->pick->masks_bad = 0u;
-    VX_CK(vx::launch_masks_hold(w->dw, &w->pick_dev->masks_bad, w->stream));
+    VX_CK(vx::launch_masks_hold(w->dw, w->d_masks + 1, w->stream));
+    VX_CK(cudaMemcpyAsync(w->d_masks, w->d_masks + 1, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                          w->stream));
+    uint32_t bad = 1u;
+    VX_CK(cudaMemcpyAsync(&bad, w->d_masks + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                          w->stream));
     VX_CK(cudaStreamSynchronize(w->stream));
-    w->masks_hold = *const_cast<volatile uint32_t *>(&w->pick->masks_bad) == 0u;
+    w->masks_hold = bad == 0u;
     return VX_OK;
 }
 
@@ -607,6 +627,7 @@ int vx_world_generate(VxWorld *w, const VxTerrainParams *t) {
     cudaError_t e = vx::launch_generate(w->dw, *t, heights, w->stream);
     cudaFreeAsync(heights, w->stream);
     VX_CK(e);
+    VX_CK(masks_rebuilt(w));
     VX_CK(cudaStreamSynchronize(w->stream));
     w->masks_hold = true;
     w->tiles_built = true;
@@ -771,6 +792,7 @@ int run_gen_plan(VxWorld *w, uint64_t seed, vx::GenPlan &plan, const std::vector
     plan.lmx = w->d_lmx;
     vx::world_masks_changed(w);
     VX_CK(vx::launch_gen_slots(w->dw, seed, plan, w->tiles_built, w->stream));
+    VX_CK(masks_rebuilt(w));
     VX_CK(cudaStreamSynchronize(w->stream));
     w->masks_hold = true;            // every mask was rebuilt
     w->tiles_built = true;
@@ -1276,7 +1298,7 @@ int vx_raycast_batch(VxWorld *w, const int32_t origin[3], const float *cams_dev,
     int rc = use_device(w);
     if (rc != VX_OK) return rc;
     VX_CK(vx::launch_raycast(w->dw, origin, cams_dev, dirs_dev, n, out_dev, hit_dev,
-                             w->masks_hold, as_stream(stream)));
+                             w->masks_hold, w->d_masks, as_stream(stream)));
     return VX_OK;
 }
 
@@ -1330,7 +1352,7 @@ int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams
             ok(cudaEventRecord(w->pick_ev[k], w->pick_in)) &&
             ok(cudaStreamWaitEvent(s, w->pick_ev[k], 0)) &&
             ok(vx::launch_raycast(w->dw, origin, cams + 3 * a, dirs + 3 * a, m, out + a,
-                                  hit + a, w->masks_hold, s)) &&
+                                  hit + a, w->masks_hold, w->d_masks, s)) &&
             ok(cudaMemcpyAsync(out_host + a, out + a, m * sizeof(VxPickHit),
                                cudaMemcpyDeviceToHost, s)) &&
             ok(cudaMemcpyAsync(hit_host + a, hit + a, m * sizeof(int32_t),

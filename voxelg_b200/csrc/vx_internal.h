@@ -116,7 +116,7 @@ cudaError_t launch_raycast_one(const DevWorld &w, const int32_t origin[3], const
                                const float dir[3], VxPickHit *out, int32_t *hit, cudaStream_t s);
 cudaError_t launch_raycast(const DevWorld &w, const int32_t origin[3], const float *cams,
                            const float *dirs, size_t n, VxPickHit *out, int32_t *hit,
-                           bool masks_hold, cudaStream_t s);
+                           bool masks_hold, const uint32_t *masks_bad, cudaStream_t s);
 // *bad = 1 (device address) when some brick with a solid voxel is not under
 // set bits of its tile, chunk and L4 words (needs tile_meta up to date)
 cudaError_t launch_masks_hold(const DevWorld &w, uint32_t *bad, cudaStream_t s);

@@ -406,6 +406,7 @@ struct PickArgs {
     DevWorld w;
     int32_t origin[3];
     float ray[6];   // single calls: camera and direction, when cams is null
+    const uint32_t *masks_bad;   // k_raycast_skip: device word, 0 where the masks hold
 };
 
 __device__ __forceinline__ bool o1_in_window(const Dims &d, const int32_t v[3],
@@ -609,9 +610,10 @@ __global__ void __launch_bounds__(128) k_raycast(PickArgs pa, const float *__res
 // clear, or an empty brick -- the walk takes them without looking: the steps
 // left to each face (the region's or the window's) sit in three 9-bit
 // counters of one word, a guard bit above each, and a step is the argmin, an
-// add and a subtraction.  Needs masks that hold for the bricks (VxWorld's
-// masks_hold); k_raycast reads the occupancy of every voxel instead, which is
-// what raycast.rs does.
+// add and a subtraction.  It goes by the masks only while they hold for the
+// bricks (VxWorld's d_masks, read when the batch runs), by bricks alone
+// otherwise; k_raycast reads the occupancy of every voxel, which is what
+// raycast.rs does, and is the faster of the two then.
 // 200,000 picks over the demo world (114 steps and 17 regions a ray): 482 us
 // voxel by voxel, 246 us here.  Rays of unlike length and place share a warp,
 // so it is bound by the lanes that wait; taking the steps of a region a few
@@ -642,6 +644,10 @@ __global__ void __launch_bounds__(128) k_raycast_skip(PickArgs pa, const float *
         const int32_t fx = s.step[0] > 0 ? -1 : 0, fy = s.step[1] > 0 ? -1 : 0,
                       fz = s.step[2] > 0 ? -1 : 0;
         const int32_t dvx = s.step[0], dvy = s.step[1] * 16, dvz = s.step[2] * 4;
+        // masks that may not hold clear no region and hide no brick
+        const bool hold = *const_cast<const volatile uint32_t *>(pa.masks_bad) == 0u;
+        const uint32_t code_bits = hold ? 3u : 0u;
+        const uint64_t any_tile = hold ? 0ull : ~0ull;
         int last = 0;              // axis of the last step (a hit always has one)
         int32_t k = 0;             // element of the walk: 4096 - k steps are left
         bool walking = false;      // phase 2: past the solids the start is in
@@ -654,8 +660,8 @@ __global__ void __launch_bounds__(128) k_raycast_skip(PickArgs pa, const float *
             if (sz >= (uint32_t)d.vz) sz -= (uint32_t)d.vz;
             const uint32_t sy = (uint32_t)ry;
             const uint32_t ti = tile_index(g, sx, sy, sz);
-            const uint64_t tw = ld_tile(w, ti);
-            const uint32_t code = (ld_tile_meta(w, ti) >> 8) & 3u;
+            const uint64_t tw = ld_tile(w, ti) | any_tile;
+            const uint32_t code = (ld_tile_meta(w, ti) >> 8) & code_bits;
             uint32_t m = 3u;       // the region is the cell of m + 1 voxels at the slot
             uint64_t occ = 0ull;   // its occupancy: a brick's, or empty
             uint32_t bi = 0u;
@@ -1049,6 +1055,7 @@ cudaError_t launch_raycast_one(const DevWorld &w, const int32_t origin[3], const
                                const float dir[3], VxPickHit *out, int32_t *hit, cudaStream_t s) {
     PickArgs pa;
     pa.w = w;
+    pa.masks_bad = nullptr;
     for (int k = 0; k < 3; ++k) {
         pa.origin[k] = origin[k];
         pa.ray[k] = cam[k];
@@ -1060,10 +1067,11 @@ cudaError_t launch_raycast_one(const DevWorld &w, const int32_t origin[3], const
 
 cudaError_t launch_raycast(const DevWorld &w, const int32_t origin[3], const float *cams,
                            const float *dirs, size_t n, VxPickHit *out, int32_t *hit,
-                           bool masks_hold, cudaStream_t s) {
+                           bool masks_hold, const uint32_t *masks_bad, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     PickArgs pa;
     pa.w = w;
+    pa.masks_bad = masks_bad;
     pa.origin[0] = origin[0]; pa.origin[1] = origin[1]; pa.origin[2] = origin[2];
     // Lanes to a ray: all 32 for the shortest time of a few, fewer as the
     // rays fill the device, and one ray a thread over the pyramid for many.
