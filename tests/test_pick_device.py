@@ -93,3 +93,86 @@ def test_captured_batch_meets_masks_that_do_not_hold(vg):
             b.check(*want)
     del graph
     dw.close()
+
+
+@pytest.mark.parametrize("n", [1, 10_000, 10_001, 25_000, 25_001, 80_000, 80_001, 100_000,
+                               100_001, 300_000])
+def test_either_side_of_every_kernel(vg, n):
+    ow = random_world(np.random.default_rng(2))
+    dw = vg.DeviceWorld(*ow.dims)
+    dw.upload(ow.a)
+    origin = (-37, 0, 70)
+    cams, dirs = rays(np.random.default_rng(n), n, ow.dims, origin)
+    b = Batch(cams, dirs)
+    b.run(dw, origin)
+    b.check(*po.raycast_batch(ow, cams, dirs, origin)[:2])
+    dw.close()
+
+
+@pytest.mark.parametrize("n", [90_000, 110_000])       # lanes to a ray, regions
+@pytest.mark.parametrize("seed", range(6))
+def test_worlds_and_windows(vg, seed, n):
+    rng = np.random.default_rng(seed)
+    ow = random_world(rng)
+    if seed % 2:        # boxes alone, with empty space of every size between
+        b = ow.a["bricks"]
+        occ = np.ascontiguousarray(b["occupancy"])
+        few = np.unpackbits(occ.view(np.uint8).reshape(-1, 8), axis=1).sum(1) < 8
+        b[few] = np.zeros(1, po.BRICK)[0]
+        ow.rebuild()
+    dw = vg.DeviceWorld(*ow.dims)
+    dw.upload(ow.a)
+    origin = (0, 0, 0) if seed == 0 else (int(rng.integers(-9000, 9000)), 0,
+                                          int(rng.integers(-9000, 9000)))
+    cams, dirs = rays(rng, n, ow.dims, origin)
+    b = Batch(cams, dirs)
+    b.run(dw, origin)
+    assert b.check(*po.raycast_batch(ow, cams, dirs, origin)[:2]) > 1000
+    dw.close()
+
+
+@pytest.mark.parametrize("n", [90_000, 110_000])
+def test_step_limit(vg, n):
+    """8192 empty voxels along x: walks end after 4096 steps, on either side of
+    a block placed at the limit, inside an empty region."""
+    dims = (2048, 16, 64)
+    ow = po.World(*dims)
+    for x in (4094, 4095, 4096, 4097):
+        ow.set_voxel(x, 8 + x - 4094, 8, 4)
+    ow.rebuild()
+    dw = vg.DeviceWorld(*dims)
+    dw.upload(ow.a)
+    y, x0 = np.meshgrid(np.arange(8, 12) + 0.5, np.arange(0, 4) + 0.5)
+    cams = np.stack([x0.ravel(), y.ravel(), np.full(x0.size, 8.5)], 1).astype(np.float32)
+    cams = np.tile(cams, (n // len(cams) + 1, 1))[:n]
+    dirs = np.tile(np.array([[1.0, 0.0, 0.0]], np.float32), (n, 1))
+    b = Batch(cams, dirs)
+    b.run(dw)
+    want = po.raycast_batch(ow, cams[:16], dirs[:16], (0, 0, 0))[:2]
+    b.check(*(np.tile(w, n // 16 + 1)[:n] for w in want))
+    dw.close()
+
+
+@pytest.mark.parametrize("name", ["tile_mask", "chunk_mask", "l4_mask"])
+def test_masks_that_do_not_hold(vg, name):
+    """raycast() reads bricks alone: uploaded masks that miss bricks must not
+    hide them, nor after updates of some bricks; generated masks hold again."""
+    rng = np.random.default_rng(3)
+    ow = random_world(rng)
+    a = {k: v.copy() for k, v in ow.a.items()}
+    a[name][:] = 0
+    dw = vg.DeviceWorld(*ow.dims)
+    dw.upload(a)
+    cams, dirs = rays(rng, 110_000, ow.dims)
+    b = Batch(cams, dirs)
+    b.run(dw)
+    assert b.check(*po.raycast_batch(ow, cams, dirs, (0, 0, 0))[:2]) > 1000
+    idx = np.arange(0, len(ow.a["bricks"]), 97, dtype=np.uint32)
+    dw.apply_dirty(idx, ow.a["bricks"][idx])
+    b.run(dw)
+    b.check(*po.raycast_batch(ow, cams, dirs, (0, 0, 0))[:2])
+    dw.generate(vg.TerrainParams(seed=9))
+    made = po.World(*ow.dims, arrays=dw.download())
+    b.run(dw)
+    b.check(*po.raycast_batch(made, cams, dirs, (0, 0, 0))[:2])
+    dw.close()
