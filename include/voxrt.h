@@ -301,10 +301,11 @@ int vx_raycast(VxWorld *w, const float cam[3], const float dir[3], const int32_t
 int vx_raycast_batch(VxWorld *w, const int32_t origin[3], const float *cams_dev,
                      const float *dirs_dev, size_t n, VxPickHit *out_dev, int32_t *hit_dev,
                      void *stream);
-/* The same over host arrays: the results are in out_host / hit_host when the
- * call returns.  Rays go to the device in chunks, each traced and its results
- * copied back while the next is on its way; results land fastest in
- * page-locked memory.  The device buffers are the world's. */
+/* The same over host arrays of any kind of memory: the results are in out_host
+ * / hit_host when the call returns.  Rays go to the device in chunks, each
+ * copied, traced and returned by one of up to eight threads (half the host's
+ * cores at most).  Calls on several threads run beside one another and beside
+ * the world's other calls; the buffers between are bounded, the world's. */
 int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams_host,
                           const float *dirs_host, size_t n, VxPickHit *out_host,
                           int32_t *hit_host);

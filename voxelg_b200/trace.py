@@ -285,16 +285,13 @@ def trace(world: DeviceWorld, rays, params: L.VxTraceParams, origin=(0, 0, 0), o
 
 
 def raycast_batch(world: DeviceWorld, cams: np.ndarray, dirs: np.ndarray, origin=(0, 0, 0)):
-    """Batched picking on the device; returns (hits PICK_DTYPE, hit flags).
-    The results are in page-locked memory, where the device writes them."""
-    torch = _torch()
+    """Batched picking on the device; returns (hits PICK_DTYPE, hit flags)."""
     n = len(cams)
     c = np.ascontiguousarray(cams, dtype=np.float32).reshape(-1)
     d = np.ascontiguousarray(dirs, dtype=np.float32).reshape(-1)
     if c.size < 3 * n or d.size < 3 * n:
         raise ValueError("raycast_batch: cams and dirs hold fewer than n x 3 floats")
-    out = torch.empty(n * 24, dtype=torch.uint8, pin_memory=True).numpy().view(L.PICK_DTYPE)
-    hit = torch.empty(n, dtype=torch.int32, pin_memory=True).numpy()
+    out, hit = np.empty(n, L.PICK_DTYPE), np.empty(n, np.int32)
     L.check(L.load().vx_raycast_batch_host(world.handle, L.i3(origin), C.c_void_p(L.ptr(c)),
                                            C.c_void_p(L.ptr(d)), n, C.c_void_p(L.ptr(out)),
                                            C.c_void_p(L.ptr(hit))))
