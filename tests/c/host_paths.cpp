@@ -328,9 +328,10 @@ cudaError_t launch_raycast_one(const DevWorld &, const int32_t *, const float ca
     return cudaSuccess;
 }
 cudaError_t launch_raycast(const DevWorld &, const int32_t *, const float *cams, const float *dirs,
-                           size_t n, VxPickHit *out, int32_t *hit, bool, const uint32_t *,
-                           cudaStream_t s) {
+                           size_t n, size_t batch, VxPickHit *out, int32_t *hit, bool,
+                           const uint32_t *, cudaStream_t s) {
     OVER;
+    g_batch_sizes.push_back(batch);
     enqueue(s, "launch_raycast", {{cams, n * 12, false}, {dirs, n * 12, false},
                                   {out, n * sizeof *out, true}, {hit, n * 4, true}});
     if (Stream *p = live(s, "launch_raycast")) g_batch_streams.insert(p->id);
@@ -439,6 +440,11 @@ void batch_memory() {
         kept.back().check("batch");
         if (g_allocs != before) wrong("a batch no larger than an earlier one allocates");
     }
+    // every launch of a batch knows the whole batch's size, which picks the kernel
+    g_batch_sizes.clear();
+    if (kept[3].run(w) != VX_OK || g_batch_sizes.size() < 2) wrong("batch");
+    for (size_t n : g_batch_sizes)
+        if (n != 200000) wrong("a chunk is launched as a batch of " + std::to_string(n));
     const size_t limit = (size_t)28 << 20;
     if (bytes_of(g_dev) - dev0 > limit) wrong("device memory kept grows with the batch");
     if (bytes_of(g_pinned) - pinned0 > limit) wrong("page-locked memory kept grows with the batch");

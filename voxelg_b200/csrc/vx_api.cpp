@@ -1328,7 +1328,7 @@ int vx_raycast_batch(VxWorld *w, const int32_t origin[3], const float *cams_dev,
     if (!vx::origin_ok(origin, "vx_raycast_batch")) return VX_ERR_INVALID;
     int rc = use_device(w);
     if (rc != VX_OK) return rc;
-    VX_CK(vx::launch_raycast(w->dw, origin, cams_dev, dirs_dev, n, out_dev, hit_dev,
+    VX_CK(vx::launch_raycast(w->dw, origin, cams_dev, dirs_dev, n, n, out_dev, hit_dev,
                              w->masks_hold, w->d_masks, as_stream(stream)));
     return VX_OK;
 }
@@ -1395,7 +1395,7 @@ int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams
                 std::memcpy(h + m * 12, dirs_host + 3 * a, m * 12);
                 r = cudaMemcpyAsync(d, h, m * kPickRayBytes, cudaMemcpyHostToDevice, s);
                 if (r == cudaSuccess)
-                    r = vx::launch_raycast(w->dw, origin, cams, dirs, m,
+                    r = vx::launch_raycast(w->dw, origin, cams, dirs, m, n,
                                            reinterpret_cast<VxPickHit *>(res),
                                            reinterpret_cast<int32_t *>(res + m * sizeof(VxPickHit)),
                                            hold, w->d_masks, s);

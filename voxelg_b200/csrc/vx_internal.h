@@ -114,8 +114,9 @@ cudaError_t launch_trace_rays(const TraceArgs &ta, const VxRay *rays, size_t n, 
 // one pick ray whose camera and direction travel in the launch parameters
 cudaError_t launch_raycast_one(const DevWorld &w, const int32_t origin[3], const float cam[3],
                                const float dir[3], VxPickHit *out, int32_t *hit, cudaStream_t s);
+// n rays of a batch of `batch` rays that other launches trace beside this one
 cudaError_t launch_raycast(const DevWorld &w, const int32_t origin[3], const float *cams,
-                           const float *dirs, size_t n, VxPickHit *out, int32_t *hit,
+                           const float *dirs, size_t n, size_t batch, VxPickHit *out, int32_t *hit,
                            bool masks_hold, const uint32_t *masks_bad, cudaStream_t s);
 // *bad = 1 (device address) when some brick with a solid voxel is not under
 // set bits of its tile, chunk and L4 words (needs tile_meta up to date)

@@ -1066,7 +1066,7 @@ cudaError_t launch_raycast_one(const DevWorld &w, const int32_t origin[3], const
 }
 
 cudaError_t launch_raycast(const DevWorld &w, const int32_t origin[3], const float *cams,
-                           const float *dirs, size_t n, VxPickHit *out, int32_t *hit,
+                           const float *dirs, size_t n, size_t batch, VxPickHit *out, int32_t *hit,
                            bool masks_hold, const uint32_t *masks_bad, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     PickArgs pa;
@@ -1080,13 +1080,17 @@ cudaError_t launch_raycast(const DevWorld &w, const int32_t origin[3], const flo
     //   8,000    38 / 39 / 48 / 70, 154     100,000  279 / 240 / 191 / 181, 182
     //   200,000  546 / 463 / 350 / 312, 246; 1,000,000  - / - / 1623 / 1367, 789
     // (one ray a thread voxel by voxel: 277, 326, 369, 383, 482, 1521)
+    // The whole batch decides, as its launches fill the device together: 200,000
+    // host rays in eight launches took 680-690 us chosen by each launch's 25,000
+    // (16 lanes) and 547-590 by regions, 1,000,000 in sixteen 2.14-2.21 ms (8
+    // lanes) and 1.91-2.10.
     auto lanes = [&](auto kernel, unsigned g) {
         kernel<<<(unsigned)((n * g + 127) / 128), 128, 0, s>>>(pa, cams, dirs, n, out, hit);
     };
-    if (n <= 10000) lanes(k_raycast<32>, 32);
-    else if (n <= 25000) lanes(k_raycast<16>, 16);
-    else if (n <= 80000) lanes(k_raycast<8>, 8);
-    else if (!masks_hold || n <= 100000) lanes(k_raycast<4>, 4);
+    if (batch <= 10000) lanes(k_raycast<32>, 32);
+    else if (batch <= 25000) lanes(k_raycast<16>, 16);
+    else if (batch <= 80000) lanes(k_raycast<8>, 8);
+    else if (!masks_hold || batch <= 100000) lanes(k_raycast<4>, 4);
     else k_raycast_skip<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(pa, cams, dirs, n, out, hit);
     return cudaGetLastError();
 }
