@@ -53,7 +53,7 @@ std::vector<Access> g_log;
 Clock g_host;                      // what the host has waited for
 size_t g_next_stream = 0, g_allocs = 0;
 long g_calls = 0, g_fail_at = 0;   // fails the g_fail_at-th call from here
-bool g_failed = false;
+bool g_failed = false, g_making = false;   // g_making: only calls that make something fail
 
 // while set, waits for streams that trace pick batches do not end
 bool g_hold = false;
@@ -62,8 +62,9 @@ std::condition_variable_any g_cv;
 std::set<size_t> g_batch_streams;
 std::vector<size_t> g_batch_sizes;  // whole-batch sizes that launch_raycast was given
 
-bool fails() {
+bool fails(bool makes = false) {
     ++g_calls;
+    if (g_making && !makes) return false;
     if (g_fail_at > 0 && --g_fail_at == 0) {
         g_failed = true;
         return true;
@@ -124,9 +125,10 @@ void forget(uint8_t *p, size_t n) {
 }
 cudaError_t give(void **p, size_t n, std::map<uint8_t *, size_t> &m) {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
-    if (fails()) return cudaErrorMemoryAllocation;
+    if (fails(true)) return cudaErrorMemoryAllocation;
     ++g_allocs;
-    uint8_t *q = static_cast<uint8_t *>(std::calloc(n ? n : 1, 1));
+    uint8_t *q = static_cast<uint8_t *>(std::malloc(n ? n : 1));
+    std::memset(q, 0xA5, n);
     m[q] = n;
     *p = q;
     return cudaSuccess;
@@ -169,6 +171,8 @@ cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
     return cudaSuccess;
 }
 cudaError_t cudaMemset(void *d, int v, size_t n) {
+    std::lock_guard<std::recursive_mutex> lk(g_mu);
+    if (fails(true)) return cudaErrorUnknown;
     std::memset(d, v, n);
     return cudaSuccess;
 }
@@ -188,7 +192,7 @@ cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t st) {
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
-    if (fails()) return cudaErrorUnknown;
+    if (fails(true)) return cudaErrorUnknown;
     Stream *p = new Stream{g_next_stream++, {}};
     g_streams.insert(p);
     *s = reinterpret_cast<cudaStream_t>(p);
@@ -223,7 +227,7 @@ cudaError_t cudaDeviceSynchronize() {
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
     std::lock_guard<std::recursive_mutex> lk(g_mu);
-    if (fails()) return cudaErrorUnknown;
+    if (fails(true)) return cudaErrorUnknown;
     Event *p = new Event;
     g_events.insert(p);
     *e = reinterpret_cast<cudaEvent_t>(p);
@@ -365,8 +369,15 @@ cudaError_t launch_dist_fields(const DevWorld &, uint8_t *, uint8_t *, uint8_t *
                                cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_edits(const DevWorld &, const uint2 *, size_t, const uint32_t *, size_t,
                          cudaStream_t) { return cudaSuccess; }
-cudaError_t launch_apply_dirty_last_wins(const DevWorld &, uint32_t *, const uint32_t *,
-                                         const VxBrick *, size_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_apply_dirty_last_wins(const DevWorld &w, uint32_t *win, const uint32_t *idx,
+                                         const VxBrick *bricks, size_t n, cudaStream_t s) {
+    OVER;
+    enqueue(s, "launch_apply_dirty", {{idx, n * 4, false}, {bricks, n * sizeof(VxBrick), false},
+                                      {win, (size_t)w.d.n_bricks * 4, true}});
+    for (size_t i = 0; i < n; ++i)
+        if (win[idx[i]] != 0u) wrong("claims of an update that are not zero");
+    return cudaSuccess;
+}
 cudaError_t launch_queue(const TraceArgs &, const VxRay *, size_t, VxHitRecord *, VxShadowRecord *,
                          const VxQueueTuning &, QueueScratch &, cudaStream_t) { return cudaSuccess; }
 cudaError_t queue_fingerprint(const VxHitRecord *, size_t, const VxShadowRecord *, QueueScratch &,
@@ -545,9 +556,10 @@ struct Frames {
     }
 };
 
-// any one call of a host frame fails: the frame says so, and the next ones use
-// only streams and events that exist and wait for what the failed one left
-void frame_errors() {
+// any one call (with making: of those that make something) of a host frame
+// fails: the frame says so, and the next ones use only streams and events that
+// exist and wait for what the failed one left
+void frames(bool making) {
     for (int warm = 0; warm < 3; ++warm) {
         long k = 0;
         for (bool more = true; more && k < 2000; ) {
@@ -557,10 +569,12 @@ void frame_errors() {
             for (int i = 0; i < warm; ++i)
                 if (f.full(w) != VX_OK) wrong("frame");
             g_failed = false;
+            g_making = making;
             g_fail_at = k;
             const int rc = (k & 1) ? f.full(w) : f.small(w);
             more = g_failed || k < 4;
             g_fail_at = 0;
+            g_making = false;
             if (g_failed != (rc != VX_OK)) wrong("frame: call " + std::to_string(k) + " fails, the frame returns " + std::to_string(rc));
             for (int i = 0; i < 3; ++i) {
                 if (f.full(w) != VX_OK) wrong("frame after a failed call");
@@ -569,8 +583,33 @@ void frame_errors() {
             }
             end_world(w);
         }
-        if (k < 10) wrong("few calls to fail");
     }
+}
+void frame_handles() { frames(true); }
+void frame_errors() { frames(false); }
+
+// the same for an update of bricks
+void update_handles() {
+    long k = 0;
+    for (bool more = true; more && k < 2000; ) {
+        ++k;
+        VxWorld *w = make_world();
+        std::vector<uint32_t> idx = {3, 9, 3};
+        std::vector<VxBrick> b(3);
+        g_failed = false;
+        g_making = true;
+        g_fail_at = k;
+        const int rc = vx_world_apply_dirty(w, idx.data(), b.data(), 3, nullptr);
+        more = g_failed;
+        g_fail_at = 0;
+        g_making = false;
+        if (g_failed != (rc != VX_OK)) wrong("update: call " + std::to_string(k) + " fails, the update returns " + std::to_string(rc));
+        for (int i = 0; i < 3; ++i)
+            if (vx_world_apply_dirty(w, idx.data(), b.data(), 3, nullptr) != VX_OK)
+                wrong("update after a failed call");
+        end_world(w);
+    }
+    if (k < 5) wrong("few calls to fail");
 }
 }  // namespace
 
@@ -579,6 +618,8 @@ int main(int argc, char **argv) {
     const std::map<std::string, void (*)()> all = {{"batch_memory", batch_memory},
                                                    {"batch_beside_others", batch_beside_others},
                                                    {"batch_errors", batch_errors},
+                                                   {"frame_handles", frame_handles},
+                                                   {"update_handles", update_handles},
                                                    {"frame_errors", frame_errors}};
     auto it = all.find(what);
     if (it == all.end()) return 2;

@@ -28,7 +28,10 @@ def exe(tmp_path_factory):
 #   other threads' batches
 # batch_errors: whichever CUDA call of a batch fails, it reports an error and
 #   the next batch is right
-@pytest.mark.parametrize("scenario", ["batch_memory", "batch_beside_others", "batch_errors"])
+# frame_handles, update_handles: whichever stream, event or buffer a host frame
+#   or an update of bricks could not make on first use, the next one makes it
+@pytest.mark.parametrize("scenario", ["batch_memory", "batch_beside_others", "batch_errors",
+                                      "frame_handles", "update_handles"])
 def test_scenario(exe, scenario):
     r = subprocess.run([str(exe), scenario], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -249,6 +249,15 @@ int use_device(VxWorld *w) {
     return VX_OK;
 }
 
+// Streams and events made on first use: each by itself, so that a call after
+// one that could not make them all makes the rest.
+cudaError_t stream_ready(cudaStream_t *s) {
+    return *s ? cudaSuccess : cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+}
+cudaError_t event_ready(cudaEvent_t *e) {
+    return *e ? cudaSuccess : cudaEventCreateWithFlags(e, cudaEventDisableTiming);
+}
+
 template <typename T>
 int ensure(T **p, size_t *cap, size_t n) {
     if (*cap >= n && *p) return VX_OK;
@@ -1251,11 +1260,16 @@ int vx_world_apply_dirty(VxWorld *w, const uint32_t *brick_idx, const VxBrick *b
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
     cudaStream_t s = stream ? as_stream(stream) : w->stream;
+    for (auto &b : w->dirty) VX_CK(event_ready(&b.done));
+    VX_CK(event_ready(&w->dirty_last));
     if (!w->d_dirty_win) {
-        VX_CK(cudaMalloc(&w->d_dirty_win, (size_t)d.n_bricks * sizeof(uint32_t)));
-        VX_CK(cudaMemset(w->d_dirty_win, 0, (size_t)d.n_bricks * sizeof(uint32_t)));
-        for (auto &b : w->dirty) VX_CK(cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming));
-        VX_CK(cudaEventCreateWithFlags(&w->dirty_last, cudaEventDisableTiming));
+        const size_t bytes = (size_t)d.n_bricks * sizeof(uint32_t);
+        uint32_t *win = nullptr;
+        VX_CK(cudaMalloc(&win, bytes));
+        const cudaError_t e = cudaMemset(win, 0, bytes);
+        if (e != cudaSuccess) cudaFree(win);
+        VX_CK(e);
+        w->d_dirty_win = win;
     }
     VxWorld::DirtyStage &b = w->dirty[w->dirty_calls & 1u];
     // the staging buffer's previous update has finished (usually long ago)
@@ -1748,15 +1762,11 @@ int enqueue_host_frame(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
     vx::FrameArgs fa = make_frame(w, cam, p);
     const size_t n = (size_t)fa.W * fa.H;
     const int buf = (int)(w->host_frames & 1u);
-    if (!w->copy_stream) {
-        VX_CK(cudaStreamCreateWithFlags(&w->copy_stream, cudaStreamNonBlocking));
-        for (auto &e : w->band_ev) VX_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        VX_CK(cudaStreamCreateWithFlags(&w->band_stream, cudaStreamNonBlocking));
-        VX_CK(cudaEventCreateWithFlags(&w->band_fork, cudaEventDisableTiming));
-    }
-    if (!w->copy_done[0]) {
-        for (auto &e : w->copy_done) VX_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
+    VX_CK(stream_ready(&w->copy_stream));
+    VX_CK(stream_ready(&w->band_stream));
+    VX_CK(event_ready(&w->band_fork));
+    for (auto &e : w->band_ev) VX_CK(event_ready(&e));
+    for (auto &e : w->copy_done) VX_CK(event_ready(&e));
     // the packed and compact forms share the device staging buffer (12 <= 16 bytes)
     const bool compact = compact_host != nullptr;
     const bool packed = packed_host != nullptr || compact;
