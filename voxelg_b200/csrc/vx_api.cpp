@@ -1753,10 +1753,9 @@ namespace {
 // rec_host / shadow_host receive the full records; or, with packed_host set,
 // each band is packed (16 bytes per pixel, shadows included) and only the
 // packed form crosses to the host.
-int enqueue_host_frame(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
-                       VxHitRecord *rec_host, VxShadowRecord *shadow_host,
-                       VxPackedRecord *packed_host, uint32_t bands,
-                       VxCompactRecord *compact_host = nullptr) {
+int enqueue_bands(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
+                  VxHitRecord *rec_host, VxShadowRecord *shadow_host, VxPackedRecord *packed_host,
+                  uint32_t bands, VxCompactRecord *compact_host) {
     static_assert(kSyncBands <= sizeof(w->band_ev) / sizeof(w->band_ev[0]), "one event per band");
     static_assert(kAsyncBands <= kSyncBands, "one event per band");
     vx::FrameArgs fa = make_frame(w, cam, p);
@@ -1838,6 +1837,19 @@ int enqueue_host_frame(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
     VX_CK(cudaEventRecord(w->copy_done[buf], w->copy_stream));
     ++w->host_frames;
     return VX_OK;
+}
+// The same; when a call of it fails, what it enqueued before is over when this
+// returns: nothing is on its way to the caller's arrays, and the next frame may
+// take the buffers.
+int enqueue_host_frame(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
+                       VxHitRecord *rec_host, VxShadowRecord *shadow_host,
+                       VxPackedRecord *packed_host, uint32_t bands,
+                       VxCompactRecord *compact_host = nullptr) {
+    const int rc = enqueue_bands(w, cam, p, rec_host, shadow_host, packed_host, bands, compact_host);
+    if (rc != VX_OK)
+        for (cudaStream_t s : {w->band_stream, w->copy_stream, w->stream})
+            if (s) cudaStreamSynchronize(s);
+    return rc;
 }
 
 int host_frame_args(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
