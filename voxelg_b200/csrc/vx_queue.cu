@@ -164,13 +164,15 @@ __global__ void __launch_bounds__(256) k_queue(QueueArgs q) {
 
 // Whole packets (refill_min 32: a warp refills when every lane is idle): a
 // warp takes 32 queue items, walks their rays to the end, then their shadow
-// rays.  No lane changes the kind of its ray inside a walk, so the walks are
-// the kind's own, without the per-iteration votes and the kind tests of
-// k_queue, whose lanes may hold any mix.  The next packet's number is asked
-// for while the current one is walked.
-// Sorted 1080p mix (3.0M rays, 1.3M shadow rays): 632 us and 531 M warp
-// instructions as lane refill at 32, 555 us and 422 M here.  At least 3 CTAs
-// of 256 (62 registers): 2, 4 and 5 measured 3, 0.5 and 2 % slower.
+// rays.  No lane changes the kind of its ray inside a walk, so a warp of one
+// kind walks in that kind's own loop, without the per-iteration votes and the
+// kind tests of k_queue, whose lanes may hold any mix; a warp of several kinds,
+// as an unsorted queue has them, in the mixed loop (one loop per kind in turn:
+// 1.1 M unsorted rays of three kinds 646 us, 445 us as lane refill, 420 us here).
+// The next packet's number is asked for while the current one is walked.
+// Sorted 1080p mix (3.1M rays, 1.3M shadow rays), the queue with its sort: 777
+// us as lane refill at 31, 690 here.  At least 3 CTAs of 256 (70 registers): 2,
+// 4 and 5 measured 3, 0.5 and 2 % slower.
 template <uint32_t FL>
 __global__ void __launch_bounds__(256, 3) k_queue_packet(QueueArgs q) {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
@@ -194,25 +196,13 @@ __global__ void __launch_bounds__(256, 3) k_queue_packet(QueueArgs q) {
             const uint32_t kind = rkind & 3u;
             Hit h;
             uint32_t ssteps = 0, sword = 0;
-            if (kind == KIND_ANY) {
-                uint32_t steps;
-                const bool occ = trace_any_ray<FL, false>(w, p, ro, ox, oy, oz, dx, dy, dz, tmax,
-                                                          steps, bytes);
-                set_miss(h);
-                h.flags = occ ? 1u : 0u;
-                h.steps = steps;
-            } else {
-                if (kind == KIND_NO_WATER)
-                    trace_no_water_ray<FL, false>(w, p, ro, ox, oy, oz, dx, dy, dz, tmax, h, bytes);
-                else
-                    trace_ray<FL, false>(w, p, ro, ox, oy, oz, dx, dy, dz, tmax, h, bytes);
-                if (q.shadow && (rkind & VX_RAY_SPAWN_SHADOW) && (h.flags & 1u)) {
-                    const ShadowRay sr = shadow_of(p, ray, ox, oy, oz, dx, dy, dz, h);
-                    const bool occ = trace_any_ray<FL, false>(w, p, ro, sr.ox, sr.oy, sr.oz, sr.dx,
-                                                              sr.dy, sr.dz, p.shadow_max_dist,
-                                                              ssteps, bytes);
-                    sword = (occ ? 1u : 0u) | (1u << 8);
-                }
+            trace_ray_of_kind<FL>(w, p, ro, kind, ox, oy, oz, dx, dy, dz, tmax, h);
+            if (q.shadow && kind != KIND_ANY && (rkind & VX_RAY_SPAWN_SHADOW) && (h.flags & 1u)) {
+                const ShadowRay sr = shadow_of(p, ray, ox, oy, oz, dx, dy, dz, h);
+                const bool occ = trace_any_ray<FL, false>(w, p, ro, sr.ox, sr.oy, sr.oz, sr.dx,
+                                                          sr.dy, sr.dz, p.shadow_max_dist, ssteps,
+                                                          bytes);
+                sword = (occ ? 1u : 0u) | (1u << 8);
             }
             store_record(q.out + ray, h);
             if (q.shadow) reinterpret_cast<uint2 *>(q.shadow)[ray] = make_uint2(ssteps, sword);
