@@ -168,11 +168,12 @@ __global__ void __launch_bounds__(256) k_queue(QueueArgs q) {
 // kind walks in that kind's own loop, without the per-iteration votes and the
 // kind tests of k_queue, whose lanes may hold any mix; a warp of several kinds,
 // as an unsorted queue has them, in the mixed loop (one loop per kind in turn:
-// 1.1 M unsorted rays of three kinds 646 us, 445 us as lane refill, 420 us here).
-// The next packet's number is asked for while the current one is walked.
+// 1.1 M unsorted rays of three kinds 646 us, 445 us as lane refill, 401 us here).
+// A warp takes a packet when it has none: one asked for ahead kept others idle
+// (90,000 unsorted rays, fewer packets than resident warps: 148 us, 97 without).
 // Sorted 1080p mix (3.1M rays, 1.3M shadow rays), the queue with its sort: 777
-// us as lane refill at 31, 690 here.  At least 3 CTAs of 256 (70 registers): 2,
-// 4 and 5 measured 3, 0.5 and 2 % slower.
+// us as lane refill at 31, 676 here (690 with a packet asked for ahead).  At
+// least 3 CTAs of 256 (70 registers): 2, 4 and 5 measured 3, 0.5 and 2 % slower.
 template <uint32_t FL>
 __global__ void __launch_bounds__(256, 3) k_queue_packet(QueueArgs q) {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
@@ -181,12 +182,11 @@ __global__ void __launch_bounds__(256, 3) k_queue_packet(QueueArgs q) {
     const Ro ro{q.ta.ro[0], q.ta.ro[1], q.ta.ro[2]};
     const VxTraceParams &p = q.ta.p;
     uint64_t bytes = 0;
-    uint32_t next = 0;
-    if (lane == 0) next = atomicAdd(q.work, 32u);
     for (;;) {
-        const uint32_t base = __shfl_sync(FULL, next, 0);
+        uint32_t base = 0;
+        if (lane == 0) base = atomicAdd(q.work, 32u);
+        base = __shfl_sync(FULL, base, 0);
         if (base >= q.n) break;
-        if (lane == 0) next = atomicAdd(q.work, 32u);
         const uint32_t slot = base + lane;
         if (slot < q.n) {
             const uint32_t ray = q.order ? __ldg(q.order + slot) : slot;
