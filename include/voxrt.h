@@ -339,7 +339,7 @@ int vx_render_primary_rows(VxWorld *w, const VxCamera *cam, const VxTraceParams 
                            void *stream);
 /* Same frame through host buffers: the records are copied to rec_host /
  * shadow_host (pinned memory recommended) before the call returns.  The
- * frame renders in six row bands, each copied while the next ones render. */
+ * frame renders in row bands, each copied while the next ones render. */
 int vx_render_primary_host(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
                            VxHitRecord *rec_host, VxShadowRecord *shadow_host);
 /* The same, for frame pipelines: enqueues the frame and returns.  Its

@@ -536,14 +536,14 @@ struct Frames {
     std::vector<VxHitRecord> rec;
     std::vector<VxShadowRecord> sh;
     std::vector<VxCompactRecord> compact;
-    Frames() {
+    explicit Frames(uint32_t width = 64, uint32_t height = 96) {
         vx_default_params(&p);
         const float pos[3] = {128.f, 32.f, 128.f};
         const int32_t o[3] = {0, 0, 0};
-        vx_camera_from_pose(pos, 0.f, 0.f, 1.f, 64, 96, o, &cam);
-        rec.resize(64 * 96);
-        sh.resize(64 * 96);
-        compact.resize(64 * 96);
+        vx_camera_from_pose(pos, 0.f, 0.f, 1.f, width, height, o, &cam);
+        rec.resize((size_t)width * height);
+        sh.resize((size_t)width * height);
+        compact.resize((size_t)width * height);
     }
     int full(VxWorld *w) { return vx_render_primary_host(w, &cam, &p, rec.data(), sh.data()); }
     int small(VxWorld *w) { return vx_render_primary_host_compact(w, &cam, &p, compact.data()); }
@@ -554,7 +554,33 @@ struct Frames {
                 return;
             }
     }
+    void check_compact() {
+        for (size_t i = 0; i < compact.size(); ++i)
+            if (compact[i].w[0] != (uint32_t)i) {
+                wrong("compact frame: record " + std::to_string(i));
+                return;
+            }
+    }
 };
+
+// frames of every split into bands and streams, one after the other on one
+// world: 4 bands on two streams, 6 on two, 4 on one, and fewer rows than bands
+void frame_sizes() {
+    VxWorld *w = make_world();
+    const uint32_t sizes[][2] = {{640, 360}, {1, 8}, {7, 1}, {1111, 1264}, {1921, 1081}, {1280, 720},
+                                 {1600, 1529}, {1600, 1530}, {2560, 1440}, {33, 9}, {1921, 1081}};
+    for (auto &q : sizes) {
+        Frames f(q[0], q[1]);
+        for (int i = 0; i < 2; ++i) {
+            std::memset(f.rec.data(), 0xFF, f.rec.size() * sizeof f.rec[0]);
+            if (f.full(w) != VX_OK) wrong("frame");
+            f.check();
+            if (f.small(w) != VX_OK) wrong("compact frame");
+            f.check_compact();
+        }
+    }
+    end_world(w);
+}
 
 // any one call (with making: of those that make something) of a host frame
 // fails: the frame says so, and the next ones use only streams and events that
@@ -618,6 +644,7 @@ int main(int argc, char **argv) {
     const std::map<std::string, void (*)()> all = {{"batch_memory", batch_memory},
                                                    {"batch_beside_others", batch_beside_others},
                                                    {"batch_errors", batch_errors},
+                                                   {"frame_sizes", frame_sizes},
                                                    {"frame_handles", frame_handles},
                                                    {"update_handles", update_handles},
                                                    {"frame_errors", frame_errors}};

@@ -28,12 +28,14 @@ def exe(tmp_path_factory):
 #   other threads' batches
 # batch_errors: whichever CUDA call of a batch fails, it reports an error and
 #   the next batch is right
+# frame_sizes: host frames of every split into bands and streams return every
+#   row and leave no access unordered
 # frame_handles, update_handles: whichever stream, event or buffer a host frame
 #   or an update of bricks could not make on first use, the next one makes it
 # frame_errors: whichever CUDA call of a host frame fails, the next frames are
 #   right and touch no buffer that work of the failed one may still use
 @pytest.mark.parametrize("scenario", ["batch_memory", "batch_beside_others", "batch_errors",
-                                      "frame_handles", "update_handles", "frame_errors"])
+                                      "frame_sizes", "frame_handles", "update_handles", "frame_errors"])
 def test_scenario(exe, scenario):
     r = subprocess.run([str(exe), scenario], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -102,7 +102,7 @@ struct VxWorld {
     std::mutex pick_mu;              // of pick_lanes alone: no batch holds it while it runs
     PickLane *pick_lanes[kPickLanes] = {};
     vx::QueueScratch qs;             // scratch of vx_queue_run / vx_queue_autotune
-    cudaEvent_t band_ev[6] = {};    // one per row band (kSyncBands at most)
+    cudaEvent_t band_ev[6] = {};    // one per row band (kBandsMax)
     cudaStream_t band_stream = nullptr;  // every other band of a synchronous host frame
     cudaEvent_t band_fork = nullptr;
     VxTuning tuning{0, {0, 0, 0, 0, 0, 0, 0}};
@@ -229,13 +229,31 @@ namespace {
 
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
-// Row bands of the host-buffer frame path.  A synchronous call copies each
-// band while the next one renders.  Pipelined calls overlap whole frames (one
-// renders while the previous one copies), so one band, i.e. the fewest
-// copies, is fastest there: 1.18 ms per 1080p frame against 1.23 ms with 8
-// bands, where the copy engine spends a few microseconds per copy.
-constexpr uint32_t kSyncBands = 6;
-constexpr uint32_t kAsyncBands = 1;
+// Row bands of the host-buffer frame path, by the bytes that go to the host.
+// Pipelined calls overlap whole frames (one renders while the previous one
+// copies), so one band, i.e. the fewest copies, is fastest there: 1.18 ms per
+// 1080p frame against 1.23 ms with 8 bands, where the copy engine spends a few
+// microseconds per copy.  A synchronous call copies each band while the next
+// ones render.  Two streams in turn shorten what the traversal bounds, since a
+// band ends with its few longest rays and the next one fills the device
+// meanwhile; but the first bands then end later, and where the copies bound the
+// frame that is what it waits for.  us, mean of three poses on a 512x256x512 /
+// 2048x256x2048 window, for 4 bands on one stream, 4 on two, 6 on two:
+//   compact 640x360    3 MB   220/254, 165/209, 183/233
+//   compact 1280x720  11 MB   309/391, 286/347, 288/358
+//   compact 1080p     25 MB   513/616, 520/631, 505/584
+//   full 1280x720     29 MB   577/588, 582/640, 593/610
+//   compact 1440p     44 MB   842/946, 887/1057, 860/967
+//   compact 2160p    100 MB  1832/1891, 1935/2276, 1873/2063
+struct BandPlan {
+    uint32_t bands;
+    bool two_streams;
+};
+constexpr uint32_t kBandsMax = 6;
+BandPlan sync_bands(size_t bytes) {
+    if (bytes >= ((size_t)28 << 20)) return {4, false};
+    return {bytes >= ((size_t)16 << 20) ? kBandsMax : 4, true};
+}
 
 // The device's word after launches that rebuilt every mask (a world whose masks
 // hold keeps it as it is).
@@ -1748,16 +1766,15 @@ namespace {
 // between two device buffers; a frame first waits, on the device, for the
 // copies of the frame two calls back that used its buffer.  Caller holds
 // w->mu.
-// One frame into host memory on the world's two streams: the traversal in
-// row bands on w->stream, each band copied on copy_stream once it is done.
+// The traversal goes to w->stream and, where the plan has two, to band_stream;
+// each band is copied on copy_stream once it is done.
 // rec_host / shadow_host receive the full records; or, with packed_host set,
 // each band is packed (16 bytes per pixel, shadows included) and only the
 // packed form crosses to the host.
 int enqueue_bands(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
                   VxHitRecord *rec_host, VxShadowRecord *shadow_host, VxPackedRecord *packed_host,
-                  uint32_t bands, VxCompactRecord *compact_host) {
-    static_assert(kSyncBands <= sizeof(w->band_ev) / sizeof(w->band_ev[0]), "one event per band");
-    static_assert(kAsyncBands <= kSyncBands, "one event per band");
+                  bool sync, VxCompactRecord *compact_host) {
+    static_assert(kBandsMax <= sizeof(w->band_ev) / sizeof(w->band_ev[0]), "one event per band");
     vx::FrameArgs fa = make_frame(w, cam, p);
     const size_t n = (size_t)fa.W * fa.H;
     const int buf = (int)(w->host_frames & 1u);
@@ -1780,7 +1797,11 @@ int enqueue_bands(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
     fa.shadow = (shadow_host || packed) ? w->hsh[buf] : nullptr;
     VX_CK(cudaStreamWaitEvent(w->stream, w->copy_done[buf], 0));
     // bands of rows (the grid form only; the persistent form renders in one go)
-    const uint32_t nb = fa.work ? 1u : bands;
+    const size_t pixel = compact ? sizeof(VxCompactRecord)
+                         : packed ? sizeof(VxPackedRecord)
+                                  : sizeof(VxHitRecord) + (shadow_host ? sizeof(VxShadowRecord) : 0);
+    const BandPlan plan = sync && !fa.work ? sync_bands(n * pixel) : BandPlan{1, false};
+    const uint32_t nb = plan.bands;
     const uint32_t band = ((fa.H + nb - 1) / nb + 7u) & ~7u;
     if (fa.ta.p.flags & VX_F_BEAM) {
         int rc = ensure(&w->beam, &w->beam_cap, (size_t)fa.bw * fa.bh);
@@ -1788,14 +1809,12 @@ int enqueue_bands(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
         fa.beam = w->beam;
         VX_CK(vx::launch_beam(fa, w->beam, w->stream));
     }
-    // Bands go to two streams in turn: a band ends with its few longest rays,
-    // and the next one fills the device meanwhile.
-    if (nb > 1) {
+    if (plan.two_streams) {
         VX_CK(cudaEventRecord(w->band_fork, w->stream));
         VX_CK(cudaStreamWaitEvent(w->band_stream, w->band_fork, 0));
     }
     for (uint32_t b = 0; b < nb; ++b) {
-        const cudaStream_t bs = (b & 1u) ? w->band_stream : w->stream;
+        const cudaStream_t bs = plan.two_streams && (b & 1u) ? w->band_stream : w->stream;
         fa.y0 = std::min(fa.H, b * band);
         fa.y1 = std::min(fa.H, (b + 1) * band);
         if (fa.work) fa.y0 = 0, fa.y1 = fa.H;
@@ -1833,7 +1852,7 @@ int enqueue_bands(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
                                   cudaMemcpyDeviceToHost, w->copy_stream));
     }
     // what follows on the world's stream follows every band
-    for (uint32_t b = 1; b < nb; b += 2) VX_CK(cudaStreamWaitEvent(w->stream, w->band_ev[b], 0));
+    for (uint32_t b = 1; b < nb && plan.two_streams; b += 2) VX_CK(cudaStreamWaitEvent(w->stream, w->band_ev[b], 0));
     VX_CK(cudaEventRecord(w->copy_done[buf], w->copy_stream));
     ++w->host_frames;
     return VX_OK;
@@ -1843,9 +1862,9 @@ int enqueue_bands(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
 // take the buffers.
 int enqueue_host_frame(VxWorld *w, const VxCamera *cam, const VxTraceParams *p,
                        VxHitRecord *rec_host, VxShadowRecord *shadow_host,
-                       VxPackedRecord *packed_host, uint32_t bands,
+                       VxPackedRecord *packed_host, bool sync,
                        VxCompactRecord *compact_host = nullptr) {
-    const int rc = enqueue_bands(w, cam, p, rec_host, shadow_host, packed_host, bands, compact_host);
+    const int rc = enqueue_bands(w, cam, p, rec_host, shadow_host, packed_host, sync, compact_host);
     if (rc != VX_OK)
         for (cudaStream_t s : {w->band_stream, w->copy_stream, w->stream})
             if (s) cudaStreamSynchronize(s);
@@ -1871,7 +1890,7 @@ int vx_render_primary_host(VxWorld *w, const VxCamera *cam, const VxTraceParams 
     int rc = host_frame_args(w, cam, p, rec_host, "vx_render_primary_host");
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
-    rc = enqueue_host_frame(w, cam, p, rec_host, shadow_host, nullptr, kSyncBands);
+    rc = enqueue_host_frame(w, cam, p, rec_host, shadow_host, nullptr, true);
     if (rc != VX_OK) return rc;
     VX_CK(cudaStreamSynchronize(w->copy_stream));
     VX_CK(cudaStreamSynchronize(w->stream));
@@ -1884,7 +1903,7 @@ int vx_render_primary_host_async(VxWorld *w, const VxCamera *cam, const VxTraceP
     int rc = host_frame_args(w, cam, p, rec_host, "vx_render_primary_host_async");
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
-    return enqueue_host_frame(w, cam, p, rec_host, shadow_host, nullptr, kAsyncBands);
+    return enqueue_host_frame(w, cam, p, rec_host, shadow_host, nullptr, false);
 }
 
 int vx_render_host_wait(VxWorld *w) {
@@ -1924,7 +1943,7 @@ int vx_render_primary_host_packed(VxWorld *w, const VxCamera *cam, const VxTrace
     if (rc == VX_OK) rc = packed_args(w, p, "vx_render_primary_host_packed");
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
-    rc = enqueue_host_frame(w, cam, p, nullptr, nullptr, out_host, kSyncBands);
+    rc = enqueue_host_frame(w, cam, p, nullptr, nullptr, out_host, true);
     if (rc != VX_OK) return rc;
     VX_CK(cudaStreamSynchronize(w->copy_stream));
     VX_CK(cudaStreamSynchronize(w->stream));
@@ -1939,7 +1958,7 @@ int vx_render_primary_host_packed_async(VxWorld *w, const VxCamera *cam,
     if (rc == VX_OK) rc = packed_args(w, p, "vx_render_primary_host_packed_async");
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
-    return enqueue_host_frame(w, cam, p, nullptr, nullptr, out_host, kAsyncBands);
+    return enqueue_host_frame(w, cam, p, nullptr, nullptr, out_host, false);
 }
 
 namespace {
@@ -1966,7 +1985,7 @@ int vx_render_primary_host_compact(VxWorld *w, const VxCamera *cam, const VxTrac
     if (rc == VX_OK) rc = compact_args(w, p, "vx_render_primary_host_compact");
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
-    rc = enqueue_host_frame(w, cam, p, nullptr, nullptr, nullptr, kSyncBands, out_host);
+    rc = enqueue_host_frame(w, cam, p, nullptr, nullptr, nullptr, true, out_host);
     if (rc != VX_OK) return rc;
     VX_CK(cudaStreamSynchronize(w->copy_stream));
     VX_CK(cudaStreamSynchronize(w->stream));
@@ -1981,7 +2000,7 @@ int vx_render_primary_host_compact_async(VxWorld *w, const VxCamera *cam,
     if (rc == VX_OK) rc = compact_args(w, p, "vx_render_primary_host_compact_async");
     if (rc != VX_OK) return rc;
     std::lock_guard<std::mutex> lk(w->mu);
-    return enqueue_host_frame(w, cam, p, nullptr, nullptr, nullptr, kAsyncBands, out_host);
+    return enqueue_host_frame(w, cam, p, nullptr, nullptr, nullptr, false, out_host);
 }
 
 namespace {
