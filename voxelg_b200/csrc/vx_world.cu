@@ -162,6 +162,15 @@ __device__ __forceinline__ uint64_t warp_child_mask(F test) {
     return (uint64_t)lo | ((uint64_t)hi << 32);
 }
 
+// the same by one thread, its 64 loads in turn
+template <typename F>
+__device__ __forceinline__ uint64_t thread_child_mask(F test) {
+    uint64_t mask = 0;
+    for (int32_t c = 0; c < 64; ++c)
+        if (test(c)) mask |= 1ull << c;
+    return mask;
+}
+
 // tile word + tile LUT from the 64 child bricks (voxel.rs:253-272, :964-972),
 // one warp
 __device__ __forceinline__ void build_tile(const DevWorld &w, int64_t ti) {
@@ -189,42 +198,43 @@ __device__ __forceinline__ void build_tile(const DevWorld &w, int64_t ti) {
     }
 }
 
-// chunk word from its (up to 64) child tiles (voxel.rs:973-981), one warp
+// chunk word from its (up to 64) child tiles (voxel.rs:973-981), one warp or
+// one thread
+template <bool THREAD = false>
 __device__ __forceinline__ void build_chunk(const DevWorld &w, int64_t ci) {
     const Dims &d = w.d;
     const int32_t cx = (int32_t)(ci % d.cx);
     const int32_t cy = (int32_t)((ci / d.cx) % d.cy);
     const int32_t cz = (int32_t)(ci / ((int64_t)d.cx * d.cy));
-    const uint64_t mask = warp_child_mask([&](int32_t c) {
+    const auto test = [&](int32_t c) {
         const int32_t tx = cx * 4 + (c & 3), ty = cy * 4 + (c >> 4), tz = cz * 4 + ((c >> 2) & 3);
         return tx < d.tx && ty < d.ty && tz < d.tz &&
                w.tile_mask[tx + (int64_t)ty * d.tx + (int64_t)tz * d.tx * d.ty] != 0ull;
-    });
-    if ((threadIdx.x & 31u) == 0u) w.chunk_mask[ci] = mask;
+    };
+    const uint64_t mask = THREAD ? thread_child_mask(test) : warp_child_mask(test);
+    if (THREAD || (threadIdx.x & 31u) == 0u) w.chunk_mask[ci] = mask;
 }
 
-// L4 word from its child chunks (voxel.rs:982-990), one warp
+// L4 word from its child chunks (voxel.rs:982-990), one warp or one thread
+template <bool THREAD = false>
 __device__ __forceinline__ void build_l4(const DevWorld &w, int64_t li) {
     const Dims &d = w.d;
     const int32_t x = (int32_t)(li % d.lx);
     const int32_t y = (int32_t)((li / d.lx) % d.ly);
     const int32_t z = (int32_t)(li / ((int64_t)d.lx * d.ly));
-    const uint64_t mask = warp_child_mask([&](int32_t c) {
+    const auto test = [&](int32_t c) {
         const int32_t cx = x * 4 + (c & 3), cy = y * 4 + (c >> 4), cz = z * 4 + ((c >> 2) & 3);
         return cx < d.cx && cy < d.cy && cz < d.cz &&
                w.chunk_mask[cx + (int64_t)cy * d.cx + (int64_t)cz * d.cx * d.cy] != 0ull;
-    });
-    if ((threadIdx.x & 31u) == 0u) w.l4_mask[li] = mask;
+    };
+    const uint64_t mask = THREAD ? thread_child_mask(test) : warp_child_mask(test);
+    if (THREAD || (threadIdx.x & 31u) == 0u) w.l4_mask[li] = mask;
 }
 
-// Every tile of a large world, one thread each: neighbouring threads read
-// neighbouring bricks, so the 64 loads in turn stream the occupancy words
-// (2048x256x2048: 27 us for 151 MB, near the copy rate; a warp per tile 57 us,
-// bound by its index arithmetic).
-__global__ void __launch_bounds__(128) k_build_tiles_stream(DevWorld w) {
+// The same words by one thread each, its 64 loads in turn: fewer instructions
+// for each word, enough where there are words to fill the device with.
+__device__ __forceinline__ void build_tile_thread(const DevWorld &w, int64_t ti) {
     const Dims &d = w.d;
-    const int64_t ti = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (ti >= d.n_tiles) return;
     const int32_t tx = (int32_t)(ti % d.tx);
     const int32_t ty = (int32_t)((ti / d.tx) % d.ty);
     const int32_t tz = (int32_t)(ti / ((int64_t)d.tx * d.ty));
@@ -241,6 +251,14 @@ __global__ void __launch_bounds__(128) k_build_tiles_stream(DevWorld w) {
             }
     w.tile_mask[ti] = mask;
     w.tile_uniform[ti] = uni ? m0 : 0;
+}
+// Every tile of a large world, one thread each: neighbouring threads read
+// neighbouring bricks, so the 64 loads in turn stream the occupancy words
+// (2048x256x2048: 27 us for 151 MB, near the copy rate; a warp per tile 57 us,
+// bound by its index arithmetic).
+__global__ void __launch_bounds__(128) k_build_tiles_stream(DevWorld w) {
+    const int64_t ti = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (ti < w.d.n_tiles) build_tile_thread(w, ti);
 }
 // one warp per cell
 __global__ void __launch_bounds__(256) k_build_tiles(DevWorld w) {
@@ -300,20 +318,25 @@ __device__ __forceinline__ BrickPos brick_pos(const Dims &d, int64_t bi) {
     return {(int32_t)(bi % d.bx), (int32_t)((bi / d.bx) % d.by),
             (int32_t)(bi / ((int64_t)d.bx * d.by))};
 }
+template <bool THREAD = false>
 __device__ __forceinline__ void dirty_tile(const DevWorld &w, int64_t bi) {
     const Dims &d = w.d;
     const BrickPos b = brick_pos(d, bi);
-    build_tile(w, (b.x / 4) + (int64_t)(b.y / 4) * d.tx + (int64_t)(b.z / 4) * d.tx * d.ty);
+    const int64_t ti = (b.x / 4) + (int64_t)(b.y / 4) * d.tx + (int64_t)(b.z / 4) * d.tx * d.ty;
+    if (THREAD) build_tile_thread(w, ti);
+    else build_tile(w, ti);
 }
+template <bool THREAD = false>
 __device__ __forceinline__ void dirty_chunk(const DevWorld &w, int64_t bi) {
     const Dims &d = w.d;
     const BrickPos b = brick_pos(d, bi);
-    build_chunk(w, (b.x / 16) + (int64_t)(b.y / 16) * d.cx + (int64_t)(b.z / 16) * d.cx * d.cy);
+    build_chunk<THREAD>(w, (b.x / 16) + (int64_t)(b.y / 16) * d.cx + (int64_t)(b.z / 16) * d.cx * d.cy);
 }
+template <bool THREAD = false>
 __device__ __forceinline__ void dirty_l4(const DevWorld &w, int64_t bi) {
     const Dims &d = w.d;
     const BrickPos b = brick_pos(d, bi);
-    build_l4(w, (b.x / 64) + (int64_t)(b.y / 64) * d.lx + (int64_t)(b.z / 64) * d.lx * d.ly);
+    build_l4<THREAD>(w, (b.x / 64) + (int64_t)(b.y / 64) * d.lx + (int64_t)(b.z / 64) * d.lx * d.ly);
 }
 
 // Any number of entries: one launch per step.
@@ -326,20 +349,29 @@ __global__ void k_dirty_scatter(DevWorld w, const uint32_t *win, const uint32_t 
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dirty_scatter(w, win, idx, bricks, i);
 }
+// an entry's words by one warp, or by one thread
+template <bool THREAD>
+__device__ __forceinline__ size_t dirty_entry() {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    return THREAD ? t : t >> 5;
+}
+template <bool THREAD>
 __global__ void __launch_bounds__(256) k_dirty_tiles(DevWorld w, uint32_t *win,
                                                      const uint32_t *idx, size_t n) {
-    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const size_t i = dirty_entry<THREAD>();
     if (i >= n) return;
-    if (win && (threadIdx.x & 31u) == 0u) win[idx[i]] = 0u;
-    dirty_tile(w, idx[i]);
+    if (win && (THREAD || (threadIdx.x & 31u) == 0u)) win[idx[i]] = 0u;
+    dirty_tile<THREAD>(w, idx[i]);
 }
+template <bool THREAD>
 __global__ void __launch_bounds__(256) k_dirty_chunks(DevWorld w, const uint32_t *idx, size_t n) {
-    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i < n) dirty_chunk(w, idx[i]);
+    const size_t i = dirty_entry<THREAD>();
+    if (i < n) dirty_chunk<THREAD>(w, idx[i]);
 }
+template <bool THREAD>
 __global__ void __launch_bounds__(256) k_dirty_l4(DevWorld w, const uint32_t *idx, size_t n) {
-    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i < n) dirty_l4(w, idx[i]);
+    const size_t i = dirty_entry<THREAD>();
+    if (i < n) dirty_l4<THREAD>(w, idx[i]);
 }
 
 // A frame's worth of entries: the same steps in one launch of one cluster,
@@ -401,6 +433,26 @@ inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t
 // CTAs of 256 threads for one warp per item
 inline unsigned warp_blocks(int64_t n) { return (unsigned)((n + 7) / 8); }
 
+// The parent words of n dirty bricks: a warp to a word while the entries are too
+// few to fill the device with one thread each, whose 64 loads in turn are a few
+// times the instructions cheaper.  Whole update, us, warp / thread: 8,000
+// entries 98-103 / 118, 16,000 167 / 175, 32,000 294 / 284, 50,000 419 / 384,
+// 200,000 1531 / 1343.
+constexpr size_t kDirtyWarpMax = 20000;
+template <bool THREAD>
+void dirty_parents_by(const DevWorld &w, uint32_t *win, const uint32_t *idx, size_t n,
+                      cudaStream_t s) {
+    const unsigned b = THREAD ? blocks_for((int64_t)n, 256) : warp_blocks((int64_t)n);
+    k_dirty_tiles<THREAD><<<b, 256, 0, s>>>(w, win, idx, n);
+    k_dirty_chunks<THREAD><<<b, 256, 0, s>>>(w, idx, n);
+    k_dirty_l4<THREAD><<<b, 256, 0, s>>>(w, idx, n);
+}
+void dirty_parents(const DevWorld &w, uint32_t *win, const uint32_t *idx, size_t n,
+                   cudaStream_t s) {
+    if (n > kDirtyWarpMax) dirty_parents_by<true>(w, win, idx, n, s);
+    else dirty_parents_by<false>(w, win, idx, n, s);
+}
+
 }  // namespace
 
 cudaError_t launch_edits(const DevWorld &w, const uint2 *ed, size_t n_edits, const uint32_t *idx,
@@ -409,10 +461,7 @@ cudaError_t launch_edits(const DevWorld &w, const uint2 *ed, size_t n_edits, con
     k_edit_voxels<<<blocks_for((int64_t)n_edits, 128), 128, 0, s>>>(w, ed, n_edits);
     const unsigned b = blocks_for((int64_t)n_bricks, 128);
     k_edit_uniform<<<b, 128, 0, s>>>(w, idx, n_bricks);
-    const unsigned bw = warp_blocks((int64_t)n_bricks);
-    k_dirty_tiles<<<bw, 256, 0, s>>>(w, nullptr, idx, n_bricks);
-    k_dirty_chunks<<<bw, 256, 0, s>>>(w, idx, n_bricks);
-    k_dirty_l4<<<bw, 256, 0, s>>>(w, idx, n_bricks);
+    dirty_parents(w, nullptr, idx, n_bricks, s);
     return launch_tile_meta(w, s);
 }
 
@@ -469,12 +518,10 @@ static cudaError_t apply_dirty(const DevWorld &w, uint32_t *win, const uint32_t 
         k_dirty_cluster<<<kDirtyCtas, kDirtyThreads, 0, s>>>(w, win, idx, bricks, (uint32_t)n);
         return launch_tile_meta(w, s);
     }
-    const unsigned b = blocks_for((int64_t)n, 128), bw = warp_blocks((int64_t)n);
+    const unsigned b = blocks_for((int64_t)n, 128);
     if (win) k_dirty_claim<<<b, 128, 0, s>>>(win, idx, n);
     k_dirty_scatter<<<b, 128, 0, s>>>(w, win, idx, bricks, n);
-    k_dirty_tiles<<<bw, 256, 0, s>>>(w, win, idx, n);
-    k_dirty_chunks<<<bw, 256, 0, s>>>(w, idx, n);
-    k_dirty_l4<<<bw, 256, 0, s>>>(w, idx, n);
+    dirty_parents(w, win, idx, n, s);
     return launch_tile_meta(w, s);
 }
 
