@@ -377,9 +377,13 @@ __global__ void __launch_bounds__(256) k_dirty_l4(DevWorld w, const uint32_t *id
 // A frame's worth of entries: the same steps in one launch of one cluster,
 // its barrier between them.  Each step is a round or two of memory latency:
 // 175 entries take 20 us, cold, against 71 us for six launches of one thread
-// per entry, most of it the 64 loads in turn and the starts and drains.
+// per entry, most of it the 64 loads in turn and the starts and drains.  The
+// cluster's 128 warps take a round for every 128 entries, and each level's
+// rounds follow one another.  Whole update, us, cluster / launches of a warp
+// per word: 32 entries 36 / 44, 175 42 / 45, 256 43 / 46, 512 54 / 49, 1,000
+// 69 / 52.
 constexpr uint32_t kDirtyCtas = 8, kDirtyThreads = 512;
-constexpr uint32_t kDirtyClusterMax = 1024;   // entries: eight rounds of the cluster's 128 warps
+constexpr uint32_t kDirtyClusterMax = 384;    // entries: three rounds
 
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;"
