@@ -649,7 +649,9 @@ int vx_wire_decode_result(const uint8_t *buf, size_t len, uint64_t *id, VxHitRec
  * vx_render_learned uses a proposal only to decide how far a verification
  * walk checks the ray before the DDA restarts past the verified cells; the
  * records equal vx_render_primary's with the same method flags and no beam,
- * except `steps` (the iterations actually executed). */
+ * except `steps`: the iterations of the ray's own walks, where one that is cut
+ * short because it has come back to a state it was in counts those it would
+ * have taken, up to the iteration cap. */
 #define VX_MLP_FLOATS 13569
 #define VX_MLP_FEATURES 80
 typedef struct VxProposal VxProposal;
@@ -703,7 +705,7 @@ typedef struct {
     uint64_t accepted;   /* verified up to the proposed distance               */
     uint64_t miss;       /* verified to the window edge / max_dist: a miss     */
     uint64_t cells;      /* verification cells stepped                         */
-    uint64_t iters;      /* DDA iterations executed                            */
+    uint64_t iters;      /* DDA iterations: the sum of the records' steps      */
     uint64_t fallback;   /* restarts that met the iteration cap (plain re-run) */
     uint64_t rays;
     float infer_ms;      /* proposal inference (0 without a proposal)          */

@@ -3,7 +3,7 @@
 // first a verification walk proves the ray's segment from the camera up to
 // the proposed start distance empty, and the DDA restarts from a point inside
 // that segment.  Records equal the plain DDA's bit for bit except `steps`
-// (iterations actually executed).
+// (iterations of its own walks; a walk cut short in a cycle counts to the cap).
 //
 // Verification.  Two empty-space distance fields (vx_distfield.cu) give, per
 // tile and per brick, the Chebyshev distance to the nearest non-empty cell of
