@@ -30,14 +30,13 @@ thread_local std::string g_last_error;
 void set_error(const std::string &msg) { g_last_error = msg; }
 }  // namespace vx
 
-// What one vx_raycast_batch_host call works with: a stream, and room for a
-// chunk of rays and results on the device and in page-locked memory, for each
-// of its threads.  Concurrent calls take one each.  A world keeps kPickLanes of
-// them between calls, at most 27 MB of device and of page-locked memory each
-// whatever the batches' sizes, and frees them with itself.
-constexpr size_t kPickThreads = 8, kPickLanes = 2, kPickChunkMin = 12288, kPickChunkMax = 65536;
+// What one vx_raycast_batch_host call works with: for each of its threads a
+// stream, room for a chunk of rays and results on the device, and page-locked
+// memory that the chunk's rays go in through and its results come out through.
+constexpr size_t kPickThreads = 8, kPickChunkMin = 12288, kPickChunkMax = 65536;
 constexpr size_t kPickRayBytes = 24, kPickHitBytes = sizeof(VxPickHit) + sizeof(int32_t);
 struct PickLane {
+    int device = 0;
     cudaStream_t stream[kPickThreads] = {};
     cudaEvent_t fork = nullptr;
     uint8_t *dev = nullptr, *host = nullptr;
@@ -59,14 +58,75 @@ struct PickLane {
         if (dev) cudaFree(dev);
         if (host) cudaFreeHost(host);
         dev = host = nullptr;
-        const size_t bytes = threads * chunk * (kPickRayBytes + kPickHitBytes);
-        e = cudaMalloc(reinterpret_cast<void **>(&dev), bytes);
+        e = cudaMalloc(reinterpret_cast<void **>(&dev),
+                       threads * chunk * (kPickRayBytes + kPickHitBytes));
         if (e == cudaSuccess)
-            e = cudaHostAlloc(reinterpret_cast<void **>(&host), bytes, cudaHostAllocDefault);
+            e = cudaHostAlloc(reinterpret_cast<void **>(&host), threads * chunk * kPickHitBytes,
+                              cudaHostAllocDefault);
         if (e == cudaSuccess) rays = threads * chunk;
         return e;
     }
 };
+// The process's idle lanes.  Concurrent calls take one each, whichever world or
+// thread they are for; kPickLanes are kept between calls, at most 27 MB on the
+// device and 15 MB page-locked each whatever the batches' sizes, and go with the
+// last world.  They outlive a world because page-locking takes about a
+// millisecond per MB: with a lane of its own, a new world's first batch of
+// 200,000 rays took 7 to 15 ms; through pieces of 64 KB each, 1 MB in all, every
+// batch of that size 1.2 ms (640 us through whole chunks).
+constexpr size_t kPickLanes = 2;
+struct PickPool {
+    std::mutex mu;                   // of the table alone: no batch holds it while it runs
+    PickLane *idle[kPickLanes] = {};
+    size_t worlds = 0;
+    PickLane *take(int device) {
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            for (PickLane *&l : idle)
+                if (l && l->device == device) {
+                    PickLane *got = l;
+                    l = nullptr;
+                    return got;
+                }
+        }
+        PickLane *made = new (std::nothrow) PickLane();
+        if (made) made->device = device;
+        return made;
+    }
+    // a lane on the calling thread's device, with nothing under way
+    void give(PickLane *lane, bool sound) {
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            for (PickLane *&l : idle)
+                if (sound && !l && worlds > 0) {
+                    l = lane;
+                    return;
+                }
+        }
+        delete lane;
+    }
+    void world_made() {
+        std::lock_guard<std::mutex> lk(mu);
+        ++worlds;
+    }
+    void world_gone() {
+        PickLane *last[kPickLanes] = {};
+        {
+            std::lock_guard<std::mutex> lk(mu);
+            if (--worlds == 0) std::swap(last, idle);
+        }
+        for (PickLane *l : last)
+            if (l) {
+                cudaSetDevice(l->device);
+                delete l;
+            }
+    }
+};
+// never destroyed: at the process's end the runtime may be gone before it
+static PickPool &pick_pool() {
+    static PickPool *p = new PickPool();
+    return *p;
+}
 
 struct VxWorld {
     int device = 0;
@@ -99,8 +159,6 @@ struct VxWorld {
     cudaStream_t copy_stream = nullptr;
     uint32_t *d_gate_idx = nullptr;  // staging of vx_project_dirty
     size_t gate_cap = 0;
-    std::mutex pick_mu;              // of pick_lanes alone: no batch holds it while it runs
-    PickLane *pick_lanes[kPickLanes] = {};
     vx::QueueScratch qs;             // scratch of vx_queue_run / vx_queue_autotune
     cudaEvent_t band_ev[6] = {};    // one per row band (kBandsMax)
     cudaStream_t band_stream = nullptr;  // every other band of a synchronous host frame
@@ -307,7 +365,6 @@ void free_world(VxWorld *w) {
     cudaFree(w->d_work);
     cudaFree(w->d_masks);
     cudaFree(w->d_gate_idx);
-    for (PickLane *l : w->pick_lanes) delete l;
     cudaFree(w->d_gen);
     cudaFree(w->d_edits);
     cudaFree(w->bdf);
@@ -556,6 +613,7 @@ int vx_world_create(const VxWorldDesc *desc, VxWorld **out) {
     VX_CKW(vx::launch_tile_meta(w->dw, w->stream));
     VX_CKW(cudaStreamSynchronize(w->stream));
 #undef VX_CKW
+    pick_pool().world_made();
     *out = w;
     return VX_OK;
 }
@@ -566,6 +624,7 @@ int vx_world_destroy(VxWorld *w) {
     if (w->stream) cudaStreamSynchronize(w->stream);
     free_world(w);
     delete w;
+    pick_pool().world_gone();
     return VX_OK;
 }
 
@@ -1393,13 +1452,7 @@ int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams
     const size_t chunks = (n + chunk - 1) / chunk;
     const size_t threads =
         std::min(std::min(std::max<size_t>(cores / 2, 1), kPickThreads), chunks);
-    PickLane *lane = nullptr;
-    {
-        std::lock_guard<std::mutex> lk(w->pick_mu);
-        for (PickLane *&l : w->pick_lanes)
-            if (!lane) std::swap(lane, l);
-    }
-    if (!lane) lane = new (std::nothrow) PickLane();
+    PickLane *lane = pick_pool().take(w->device);
     if (!lane) {
         vx::set_error("vx_raycast_batch_host: out of memory");
         return VX_ERR_OOM;
@@ -1412,8 +1465,8 @@ int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams
         std::atomic<size_t> next{0};
         std::atomic<int> failed{(int)cudaSuccess};
         auto work = [&](size_t t) {
-            const size_t room = chunk * (kPickRayBytes + kPickHitBytes);
-            uint8_t *d = lane->dev + t * room, *h = lane->host + t * room;
+            uint8_t *d = lane->dev + t * chunk * (kPickRayBytes + kPickHitBytes);
+            uint8_t *h = lane->host + t * chunk * kPickHitBytes;
             const cudaStream_t s = lane->stream[t];
             cudaError_t r = cudaSetDevice(w->device);
             if (r == cudaSuccess) r = cudaStreamWaitEvent(s, lane->fork, 0);
@@ -1422,7 +1475,7 @@ int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams
                 if (k >= chunks) break;
                 const size_t a = k * chunk, m = std::min(chunk, n - a);
                 float *cams = reinterpret_cast<float *>(d), *dirs = cams + 3 * m;
-                uint8_t *res = d + m * kPickRayBytes, *hres = h + m * kPickRayBytes;
+                uint8_t *res = d + m * kPickRayBytes;
                 std::memcpy(h, cams_host + 3 * a, m * 12);
                 std::memcpy(h + m * 12, dirs_host + 3 * a, m * 12);
                 r = cudaMemcpyAsync(d, h, m * kPickRayBytes, cudaMemcpyHostToDevice, s);
@@ -1432,7 +1485,7 @@ int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams
                                            reinterpret_cast<int32_t *>(res + m * sizeof(VxPickHit)),
                                            hold, w->d_masks, s);
                 if (r == cudaSuccess)
-                    r = cudaMemcpyAsync(hres, res, m * kPickHitBytes, cudaMemcpyDeviceToHost, s);
+                    r = cudaMemcpyAsync(h, res, m * kPickHitBytes, cudaMemcpyDeviceToHost, s);
                 // the pages that the results go to, while the device traces
                 volatile uint8_t *page = reinterpret_cast<uint8_t *>(out_host + a);
                 for (size_t b = 0; b < m * sizeof(VxPickHit); b += 4096) page[b] = 0;
@@ -1442,8 +1495,8 @@ int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams
                 const cudaError_t end = cudaStreamSynchronize(s);
                 if (r == cudaSuccess) r = end;
                 if (r != cudaSuccess) break;
-                std::memcpy(out_host + a, hres, m * sizeof(VxPickHit));
-                std::memcpy(hit_host + a, hres + m * sizeof(VxPickHit), m * sizeof(int32_t));
+                std::memcpy(out_host + a, h, m * sizeof(VxPickHit));
+                std::memcpy(hit_host + a, h + m * sizeof(VxPickHit), m * sizeof(int32_t));
             }
             int none = (int)cudaSuccess;
             if (r != cudaSuccess) failed.compare_exchange_strong(none, (int)r);
@@ -1461,15 +1514,7 @@ int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams
             if (t.joinable()) t.join();
         e = (cudaError_t)failed.load();
     }
-    if (e == cudaSuccess) {
-        std::lock_guard<std::mutex> lk(w->pick_mu);
-        for (PickLane *&l : w->pick_lanes)
-            if (!l) {
-                std::swap(lane, l);
-                break;
-            }
-    }
-    delete lane;                     // after an error, or when enough are kept
+    pick_pool().give(lane, e == cudaSuccess);
     VX_CK(e);
     return VX_OK;
 }
