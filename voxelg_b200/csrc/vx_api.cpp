@@ -212,7 +212,7 @@ struct VxWorld {
     // host's flag picks the faster kernel; the device's word (d_masks[0],
     // nonzero where the masks may not hold) is what the kernel goes by, so a
     // batch that was captured in a graph or waits on another stream meets the
-    // world as it then is.  d_masks[1] is the check's own.
+    // world as it then is.  d_masks[1] is the check's own; both lie behind d_work.
     std::atomic<bool> masks_hold{true};
     uint32_t *d_masks = nullptr;
     bool tiles_built = true;         // tile words and LUT bytes are the library's, for every tile
@@ -363,7 +363,6 @@ void free_world(VxWorld *w) {
     cudaFree(w->sh);
     if (w->pick) cudaFreeHost(w->pick);
     cudaFree(w->d_work);
-    cudaFree(w->d_masks);
     cudaFree(w->d_gate_idx);
     cudaFree(w->d_gen);
     cudaFree(w->d_edits);
@@ -594,10 +593,9 @@ int vx_world_create(const VxWorldDesc *desc, VxWorld **out) {
     VX_CKW(cudaMalloc(&w->dw.oob, sizeof(unsigned long long)));
     VX_CKW(cudaMemsetAsync(w->dw.oob, 0, sizeof(unsigned long long), w->stream));
     VX_CKW(cudaMalloc(&w->d_stats, 4 * sizeof(unsigned long long)));
-    VX_CKW(cudaMalloc(&w->d_work, 2 * sizeof(uint32_t)));
-    VX_CKW(cudaMemsetAsync(w->d_work, 0, 2 * sizeof(uint32_t), w->stream));
-    VX_CKW(cudaMalloc(&w->d_masks, 2 * sizeof(uint32_t)));
-    VX_CKW(cudaMemsetAsync(w->d_masks, 0, 2 * sizeof(uint32_t), w->stream));
+    VX_CKW(cudaMalloc(&w->d_work, 4 * sizeof(uint32_t)));
+    VX_CKW(cudaMemsetAsync(w->d_work, 0, 4 * sizeof(uint32_t), w->stream));
+    w->d_masks = w->d_work + 2;
     VX_CKW(cudaHostAlloc(reinterpret_cast<void **>(&w->pick), sizeof(VxWorld::PickBox),
                          cudaHostAllocMapped));
     VX_CKW(cudaHostGetDevicePointer(reinterpret_cast<void **>(&w->pick_dev), w->pick, 0));
