@@ -140,7 +140,7 @@ cudaError_t launch_bricks_to_aos(const DevWorld &w, VxBrick *aos, int64_t first,
 // source chunks in (z, x) order; cols / srcs hold (x, z) pairs.  A window
 // plan (window == true) generates every slot of the window whose lower
 // corner is world chunk (ox, 0, oz) and derives all of that on the device:
-// job b is slot (b % SX, b / SX % SY, b / (SX SY)), column k the slot column
+// job b is slot (b % SX, b / (SX SZ), b / SX % SZ), column k the slot column
 // (k % SX, k / SX), source k world chunk (ox - 1 + k % (SX + 2),
 // oz - 1 + k / (SX + 2)).  colw has 1024 words per column chunk, prims
 // gen_prim_bytes_per_src() bytes and hdr 12 ints per source chunk.  The
@@ -172,7 +172,6 @@ cudaError_t launch_generate(const DevWorld &w, const VxTerrainParams &t, int16_t
                             cudaStream_t s);
 // chunk and L4 words and tile_meta, after the tiles' where `tiles`
 cudaError_t launch_rebuild_pyramid(const DevWorld &w, bool tiles, cudaStream_t s);
-// the brick and tile distance fields of w (tmp: n_bricks bytes of scratch)
 // a frame's records (and shadow records, or nullptr) [first, first + n) in
 // the 16-byte packed form (vx_pack.cu)
 // records [first, first + n) as VxCompactRecord; a record the form cannot
@@ -183,6 +182,7 @@ cudaError_t launch_pack_compact(const VxHitRecord *rec, const VxShadowRecord *sh
 cudaError_t launch_pack(const VxHitRecord *rec, const VxShadowRecord *sh, size_t first, size_t n,
                         const int32_t ro[3], uint32_t wx, uint32_t wy, VxPackedRecord *out,
                         cudaStream_t s);
+// the brick and tile distance fields of w (tmp: n_bricks bytes of scratch)
 cudaError_t launch_dist_fields(const DevWorld &w, uint8_t *bdf, uint8_t *tdf, uint8_t *tmp,
                                cudaStream_t s);
 // tile_meta of every tile from the masks and the tile LUT
@@ -199,7 +199,7 @@ cudaError_t launch_apply_dirty(const DevWorld &w, const uint32_t *idx, const VxB
                                size_t n, cudaStream_t s);
 
 // Scratch of one ray-queue configuration (owned by a world or a graph):
-// work counters, coherence-sort keys / permutation / histogram, fingerprint.
+// work counters, the coherence sort's places, order and counts, fingerprint.
 struct QueueScratch {
     uint32_t *work = nullptr;
     uint2 *place = nullptr;       // coherence sort: each ray's bucket and place in it

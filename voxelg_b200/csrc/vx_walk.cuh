@@ -627,7 +627,10 @@ __device__ __forceinline__ SeenKey seen_key(const Walk &k, bool keeps_t) {
 // words of the state kept across the loop 2-3 %, the loop copied for the
 // stretches 5-9 %.
 // c2 frame (2048x256x2048, 1920x1080, some rays of 1024 steps): 487 us before,
-// 362 us with it.
+// 362 us with it; 320x180 of the same 109 and 68 (mean of four poses).  Where no
+// ray cycles it costs up to 3 % (640x360, LUT and LOD: 69 us before, 71 with it;
+// 2160p on 512x256x512: 744 and 749); looks from iteration 240 or 360 on, or every
+// 120 or 250, cost the same and find less.
 constexpr uint32_t kSeenFirst = 180, kSeenEvery = 60;
 template <uint32_t FL, bool STATS, int KNOWN>
 __device__ __forceinline__ int walk_to_end(const DevWorld &w, const Geo &g, const VxTraceParams &p,
@@ -706,9 +709,10 @@ __device__ __forceinline__ void trace_no_water_ray(const DevWorld &w, const VxTr
 // A generic ray of any kind (VxRay: 1 any hit, 2 no water, else trace).  The
 // lanes of a warp may hold different kinds; they then walk together, the kind
 // decided in the loop.  A loop per kind one after the other costs such a warp
-// the longest ray of each kind in turn (2 M rays of three kinds: 710 us, 494 us
-// together; 1,000 rays: 42 and 30 us).  Warps of one kind keep that kind's
-// loop, which is 4-15 % faster than the mixed one.
+// the longest ray of each kind in turn (2 M rays of three kinds: 691 us, 469 us
+// together; 1,000 rays: 45 and 30 us).  Warps of one kind keep that kind's
+// loop, which is 4-15 % faster than the mixed one (2 M rays of kind 1: 346 us as
+// the launch's only loop, 354 here; kinds 0 and 2 420 / 414 and 470 / 451).
 template <uint32_t FL>
 __device__ __forceinline__ void trace_ray_of_kind(const DevWorld &w, const VxTraceParams &p, Ro ro,
                                                   uint32_t kind, float o0, float o1, float o2,
