@@ -305,7 +305,8 @@ int vx_raycast_batch(VxWorld *w, const int32_t origin[3], const float *cams_dev,
  * / hit_host when the call returns.  Rays go to the device in chunks, each
  * copied, traced and returned by one of up to eight threads (half the host's
  * cores at most).  Calls on several threads run beside one another and beside
- * the world's other calls; the buffers between are bounded, the world's. */
+ * the world's other calls.  The buffers between are bounded, shared by the
+ * process's worlds, and freed with the last of them. */
 int vx_raycast_batch_host(VxWorld *w, const int32_t origin[3], const float *cams_host,
                           const float *dirs_host, size_t n, VxPickHit *out_host,
                           int32_t *hit_host);

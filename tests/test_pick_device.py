@@ -176,3 +176,43 @@ def test_masks_that_do_not_hold(vg, name):
     b.run(dw)
     b.check(*po.raycast_batch(made, cams, dirs, (0, 0, 0))[:2])
     dw.close()
+
+
+def test_host_batches_on_threads(vg):
+    """Batches of several sizes at once on two worlds, each from its own thread,
+    single picks between them: every result is the ray's own."""
+    import threading
+    rng = np.random.default_rng(7)
+    worlds = []
+    for seed in (4, 5):
+        ow = random_world(np.random.default_rng(seed))
+        dw = vg.DeviceWorld(*ow.dims)
+        dw.upload(ow.a)
+        worlds.append((ow, dw))
+    jobs, wrong = [], []
+    for k, n in enumerate((150_001, 40_000, 12_289, 100, 150_001, 1)):
+        ow, dw = worlds[k % 2]
+        cams, dirs = rays(rng, n, ow.dims)
+        jobs.append((dw, cams, dirs, *po.raycast_batch(ow, cams, dirs, (0, 0, 0))[:2]))
+
+    def work(job):
+        dw, cams, dirs, want, want_hit = job
+        for _ in range(6):
+            hits, found = vg.raycast_batch(dw, cams, dirs)
+            sel = want_hit != 0
+            if not (np.array_equal(found, want_hit)
+                    and np.array_equal(hits["voxel"][sel], want["voxel"][sel])
+                    and np.array_equal(hits["normal"][sel], want["normal"][sel])):
+                wrong.append(len(cams))
+            one = vg.raycast(cams[0], dirs[0], dw)
+            if (one is not None) != bool(want_hit[0]):
+                wrong.append("single")
+
+    threads = [threading.Thread(target=work, args=(j,)) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    for _, dw in worlds:
+        dw.close()
